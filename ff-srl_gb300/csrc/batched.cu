@@ -69,6 +69,7 @@ struct ffsrl_batch {
     int* d_cnt0 = nullptr;        // static per-vertex contribution counts
     int* d_tet_orig = nullptr;    // record -> model tet id
     int* d_edge_orig = nullptr;   // record -> model edge id
+    PartRec* d_part = nullptr; int* d_vmap = nullptr; unsigned* d_xch = nullptr;  // split envs
     uint2* d_conn_idx = nullptr; float4* d_conn_bar = nullptr; unsigned char* d_conn_vert = nullptr;
     long long* d_pend = nullptr; int* d_pcnt = nullptr;  // pending connector corrections, kept between steps
     unsigned long long* d_wide = nullptr;  // fixed-point side accumulator [3V], zero between uses
@@ -80,7 +81,10 @@ struct ffsrl_batch {
     size_t dyn_budget = 0;
     // classes
     struct Class {
-        int mode, block, max_nv, grid, members;
+        int mode;          // storage of an undivided env of the class
+        int block, max_nv, grid, members;
+        int split = 1;     // blocks that step one env (a cluster); max_nv is then a part's
+        int env_nv = 0;    // largest env vertex count
         int prefetch = 0;  // L1 prefetch of the next tet record (autotuned)
         int tri_cap = 0;   // surface triangles kept in shared memory per env (0: read from L2)
         size_t smem, scratch_stride, scratch_offset;
@@ -127,7 +131,7 @@ void free_batch(ffsrl_batch* b) {
     cudaFree(b->d_tet_vs); cudaFree(b->d_edge_idx); cudaFree(b->d_edge_la); cudaFree(b->d_tri_idx);
     cudaFree(b->d_work); cudaFree(b->d_status); cudaFree(b->d_scratch);
     cudaFree(b->d_state64); cudaFree(b->d_cnt0); cudaFree(b->d_tet_orig);
-    cudaFree(b->d_edge_orig);
+    cudaFree(b->d_edge_orig); cudaFree(b->d_part); cudaFree(b->d_vmap); cudaFree(b->d_xch);
     cudaFree(b->d_conn_idx); cudaFree(b->d_conn_bar); cudaFree(b->d_conn_vert); cudaFree(b->d_pend); cudaFree(b->d_pcnt);
     cudaFree(b->d_wide); cudaFree(b->d_nhd); cudaFree(b->d_tet_ed2);
     for (auto& l : b->lanes) {
@@ -142,12 +146,18 @@ void free_batch(ffsrl_batch* b) {
     delete b;
 }
 
-int default_block(int max_nv, int mode) {
+// Threads of an undivided env's block.  `few`: the plan has at most one env per SM, so that a
+// block has its SM to itself and more warps shorten it; with more envs, smaller blocks share
+// an SM better (2048 mixed envs, fast arithmetic: 17.1 ms with 256 threads up to 1,024
+// vertices, 18.2 with 512).  768 threads are the most whose registers hold the tet loop: of
+// 80 envs of 10k-19k tets a step took 8.96 ms (reference) and 4.20 ms (fast), against 9.69
+// and 4.74 with 1,024 threads, which spill.  With the sums in global scratch (mode 1) the
+// 46,640-tet ellipsoid took 37.1 ms with 512 threads, 42.9 with 1,024.
+int default_block(int max_nv, int mode, bool few) {
     if (mode == 2) return 256;
-    if (max_nv <= 256) return 128;
-    if (max_nv <= 1024) return 256;
-    if (max_nv <= 2560) return 512;
-    return 1024;
+    if (max_nv > 2560) return mode == 1 ? 512 : 768;
+    if (max_nv > 1024 || few) return 512;
+    return max_nv <= 256 ? 128 : 256;
 }
 
 template <class R> int32_t launch_class(ffsrl_batch* b, const ffsrl_batch::Class& c, const int* work, int nwork,
@@ -159,6 +169,24 @@ kern_f kernel_f(const ffsrl_batch* b, int block, int mode, int prefetch) {
     if (b->accum != FFSRL_ACC_FIXED) return prefetch ? nullptr : pick_ref_study(b->accum, block, mode);
     if (b->arith == FFSRL_ARITH_FAST) return pick_fast_fixed(block, mode, prefetch, b->params.flags);
     return pick_ref_fixed(block, mode, prefetch, b->params.flags);
+}
+// The kernel that steps one env with a cluster of blocks (float32 fixed-point plans)
+kern_f split_f(const ffsrl_batch* b, int block) {
+    return b->arith == FFSRL_ARITH_FAST ? pick_fast_split(block, b->params.flags) : pick_ref_split(block, b->params.flags);
+}
+// A launch of `envs` clusters, one env each at a time
+cudaLaunchConfig_t cluster_config(const ffsrl_batch::Class& c, int envs, cudaLaunchAttribute* at, cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)c.split;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(envs * c.split));
+    cfg.blockDim = dim3((unsigned)c.block);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
 }
 const void* kernel_ptr(const ffsrl_batch* b, int block, int mode, int prefetch) {
     if (b->precision == 64) return prefetch ? nullptr : (const void*)pick_ref_f64(block, mode);
@@ -191,6 +219,7 @@ Dev<float> make_dev_f(ffsrl_batch* b) {
     D.tet_lambda = b->dm.tetrahedron_lambda; D.edge_lambda = b->dm.edge_lambda;
     D.env_status = b->d_status;
     D.cnt0 = b->d_cnt0; D.tet_orig = b->d_tet_orig; D.edge_orig = b->d_edge_orig;
+    D.part = b->d_part; D.vmap = b->d_vmap; D.xch = b->d_xch;
     D.nhd = b->d_nhd; D.wide = b->d_wide; D.bound = b->bound;
     D.tet_ed = b->d_tet_ed; D.tet_ed2 = b->d_tet_ed2; D.compact = b->compact;
     D.fold = b->d_tet_ed != nullptr || b->d_tet_ed2 != nullptr;
@@ -209,11 +238,18 @@ Dev<float> make_dev_f(ffsrl_batch* b) {
 
 template <> int32_t launch_class<float>(ffsrl_batch* b, const ffsrl_batch::Class& c, const int* work, int nwork,
                                         int* counter, unsigned char* scratch, int nsteps, cudaStream_t s) {
-    kern_f k = kernel_f(b, c.block, c.mode, c.prefetch);
+    kern_f k = c.split > 1 ? split_f(b, c.block) : kernel_f(b, c.block, c.mode, c.prefetch);
     if (!k) return fail(FFSRL_ERR_UNSUPPORTED, "ffsrl_batch: no kernel for block/mode");
     Dev<float> D = make_dev_f(b);
     int grid = std::min(c.grid, nwork);
     if (grid <= 0) return FFSRL_OK;
+    if (c.split > 1) {
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t cfg = cluster_config(c, grid, at, s);
+        FFSRL_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, (const Dev<float>)D, work, nwork, counter, nsteps, (unsigned char*)nullptr,
+                                          0ll, c.max_nv, 0, c.tri_cap));
+        return FFSRL_OK;
+    }
     k<<<grid, c.block, c.smem, s>>>(D, work, nwork, counter, nsteps, scratch + c.scratch_offset,
                                     (long long)c.scratch_stride, c.max_nv, c.prefetch == 1 ? 1 : 0, c.tri_cap);
     FFSRL_LAUNCH_CHECK("ffsrl_batch: step kernel");
@@ -235,6 +271,7 @@ template <> int32_t launch_class<double>(ffsrl_batch* b, const ffsrl_batch::Clas
     D.lap_radius = F.lap_radius; D.in_collision = F.in_collision; D.tet_lambda = F.tet_lambda;
     D.edge_lambda = F.edge_lambda; D.env_status = F.env_status; D.flags = F.flags; D.substeps = F.substeps;
     D.cnt0 = F.cnt0; D.tet_orig = F.tet_orig; D.edge_orig = F.edge_orig;
+    D.part = nullptr; D.vmap = nullptr; D.xch = nullptr;
     D.nhd = F.nhd; D.wide = F.wide; D.bound = F.bound; D.pend = nullptr; D.pcnt = nullptr;
     D.conn_idx = nullptr; D.conn_bar = nullptr; D.conn_vert = nullptr;
     D.tet_ed = F.tet_ed; D.tet_ed2 = nullptr; D.compact = 0; D.fold = F.fold;
@@ -321,11 +358,266 @@ void bank_regroup(std::vector<int>& ord, int corners, VertFn vert, KeyFn key, in
     ord.swap(out);
 }
 
-// Block size of a class: the instantiation, its shared-memory allowance and the grid
-// from the runtime's occupancy calculator.
 constexpr int kLanes = 2;
 
+// ---- envs split over a cluster of blocks ---------------------------------------------
+// Cluster sizes in use (where the device has room for one): those that fill most of the
+// 152 SMs when every SM holds one block -- 76, 46, 36, 23, 15 and 7 of them fit at a time --
+// and few enough that the classes they form run beside one another.
+constexpr int kSplits[] = {2, 3, 4, 6, 9, 16};
+constexpr int kMaxSplit = 16;
+// A part has at least this many tets: the 800-tet beam takes 387 us a step in 6 to 8 parts,
+// 410 in 12, 470 undivided.
+constexpr int kMinPartTets = 100;
+
+// One env's parts, offsets relative to the env's records and to vmap / xch
+struct Split {
+    std::vector<PartRec> parts;
+    std::vector<int> tets, edges, tris;  // the env's records (env-relative) in part order
+    std::vector<uint2> tet_ids, tri_ids; // their vertex ids in their parts (and the triangles' hole bits)
+    std::vector<unsigned> edge_ids;
+    std::vector<int> vmap;
+    std::vector<unsigned> xch;
+    int max_loc = 0;
+};
+
+// Shares out one env's records among G parts of equal tet counts: recursive bisection of
+// the tets' centroids along the longest side.  A vertex belongs to the part that holds most
+// of its tets; an edge or a triangle goes to a part that already holds its vertices where
+// there is one, else to its first vertex's owner.
+Split split_env(int G, int nv, const float* x, const std::vector<uint2>& tet_idx, int t0, int nt,
+                const std::vector<unsigned>& edge_idx, int e0, int ne, const std::vector<uint2>& tri_idx, int f0, int nf) {
+    Split S;
+    auto corners = [](uint2 ix, int* l) {
+        l[0] = ix.x & 0xffff; l[1] = ix.x >> 16; l[2] = ix.y & 0xffff; l[3] = ix.y >> 16;
+    };
+    std::vector<float> cen(3 * (size_t)nt);
+    for (int t = 0; t < nt; ++t) {
+        int l[4];
+        corners(tet_idx[t0 + t], l);
+        for (int d = 0; d < 3; ++d) {
+            const float c = x[3 * l[0] + d] + x[3 * l[1] + d] + x[3 * l[2] + d] + x[3 * l[3] + d];
+            cen[3 * (size_t)t + d] = std::isfinite(c) ? c : 0.0f;  // (a NaN has no place in an order)
+        }
+    }
+    std::vector<int> ord(nt), part_of(nt);
+    std::iota(ord.begin(), ord.end(), 0);
+    struct Range { int lo, hi, p, g; };
+    std::vector<Range> todo{{0, nt, 0, G}};
+    while (!todo.empty()) {
+        const Range r = todo.back();
+        todo.pop_back();
+        if (r.g == 1) {
+            for (int i = r.lo; i < r.hi; ++i) part_of[ord[i]] = r.p;
+            continue;
+        }
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        for (int i = r.lo; i < r.hi; ++i)
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = std::min(lo[d], cen[3 * (size_t)ord[i] + d]);
+                hi[d] = std::max(hi[d], cen[3 * (size_t)ord[i] + d]);
+            }
+        int ax = 0;
+        for (int d = 1; d < 3; ++d)
+            if (hi[d] - lo[d] > hi[ax] - lo[ax]) ax = d;
+        const int mid = r.lo + (int)((int64_t)(r.hi - r.lo) * (r.g / 2) / r.g);
+        std::nth_element(ord.begin() + r.lo, ord.begin() + mid, ord.begin() + r.hi, [&](int a, int c) {
+            const float u = cen[3 * (size_t)a + ax], v = cen[3 * (size_t)c + ax];
+            return u != v ? u < v : a < c;
+        });
+        todo.push_back({r.lo, mid, r.p, r.g / 2});
+        todo.push_back({mid, r.hi, r.p + r.g / 2, r.g - r.g / 2});
+    }
+    std::vector<int> count((size_t)G * nv, 0), owner(nv, 0);
+    for (int t = 0; t < nt; ++t) {
+        int l[4];
+        corners(tet_idx[t0 + t], l);
+        for (int k = 0; k < 4; ++k) count[(size_t)part_of[t] * nv + l[k]]++;
+    }
+    for (int v = 0; v < nv; ++v)
+        for (int p = 1; p < G; ++p)
+            if (count[(size_t)p * nv + v] > count[(size_t)owner[v] * nv + v]) owner[v] = p;
+    // held[p][v]: part p holds vertex v
+    std::vector<unsigned char> held((size_t)G * nv);
+    for (size_t i = 0; i < held.size(); ++i) held[i] = count[i] > 0;
+    for (int v = 0; v < nv; ++v) held[(size_t)owner[v] * nv + v] = 1;
+    auto home = [&](const int* l, int n) {
+        for (int k = 0; k < n; ++k) {
+            bool all = true;
+            for (int j = 0; j < n; ++j) all = all && held[(size_t)owner[l[k]] * nv + l[j]];
+            if (all) return owner[l[k]];
+        }
+        for (int j = 0; j < n; ++j) held[(size_t)owner[l[0]] * nv + l[j]] = 1;
+        return owner[l[0]];
+    };
+    std::vector<int> edge_of(ne), tri_of(nf);
+    for (int e = 0; e < ne; ++e) {
+        const int l[2] = {(int)(edge_idx[e0 + e] & 0xffff), (int)(edge_idx[e0 + e] >> 16)};
+        edge_of[e] = home(l, 2);
+    }
+    for (int f = 0; f < nf; ++f) {
+        const uint2 ix = tri_idx[f0 + f];
+        const int l[3] = {(int)(ix.x & 0xffff), (int)(ix.x >> 16), (int)(ix.y & 0xffff)};
+        tri_of[f] = home(l, 3);
+    }
+    std::vector<int> copies(nv, 0);
+    for (int p = 0; p < G; ++p)
+        for (int v = 0; v < nv; ++v) copies[v] += held[(size_t)p * nv + v];
+    // local ids: owned vertices, then the halo
+    std::vector<int> local((size_t)G * nv, -1);
+    S.parts.resize(G);
+    for (int p = 0; p < G; ++p) {
+        PartRec& P = S.parts[p];
+        P = PartRec{};
+        P.map0 = (int)S.vmap.size();
+        for (int inner = 0; inner < 2; ++inner) {  // boundary vertices, which other parts hold too, first
+            for (int v = 0; v < nv; ++v)
+                if (owner[v] == p && (copies[v] == 1) == (inner == 1)) { local[(size_t)p * nv + v] = P.n_own++; S.vmap.push_back(v); }
+            if (!inner) P.n_bnd = P.n_own;
+        }
+        P.n_loc = P.n_own;
+        for (int v = 0; v < nv; ++v)
+            if (owner[v] != p && held[(size_t)p * nv + v]) { local[(size_t)p * nv + v] = P.n_loc++; S.vmap.push_back(v); }
+        S.max_loc = std::max(S.max_loc, P.n_loc);
+    }
+    for (int p = 0; p < G; ++p) {
+        PartRec& P = S.parts[p];
+        const int* loc = &local[(size_t)p * nv];
+        auto word = [&](int q, int v) { return ((unsigned)q << 16) | (unsigned)local[(size_t)q * nv + v]; };
+        P.x0 = (int)S.xch.size();
+        for (int i = P.n_own; i < P.n_loc; ++i) {
+            const int v = S.vmap[P.map0 + i];
+            S.xch.push_back(word(owner[v], v));
+        }
+        std::vector<unsigned> first{0};
+        for (int i = 0; i < P.n_bnd; ++i) {
+            const int v = S.vmap[P.map0 + i];
+            for (int q = 0; q < G; ++q)
+                if (q != p && held[(size_t)q * nv + v]) { S.xch.push_back(word(q, v)); ++P.n_in; }
+            first.push_back((unsigned)P.n_in);
+        }
+        S.xch.insert(S.xch.end(), first.begin(), first.end());
+        P.t0 = (int)S.tets.size(); P.e0 = (int)S.edges.size(); P.f0 = (int)S.tris.size();
+        for (int t = 0; t < nt; ++t)
+            if (part_of[t] == p) {
+                int l[4];
+                corners(tet_idx[t0 + t], l);
+                S.tets.push_back(t);
+                S.tet_ids.push_back(make_uint2((unsigned)loc[l[0]] | ((unsigned)loc[l[1]] << 16),
+                                               (unsigned)loc[l[2]] | ((unsigned)loc[l[3]] << 16)));
+            }
+        for (int e = 0; e < ne; ++e)
+            if (edge_of[e] == p) {
+                S.edges.push_back(e);
+                S.edge_ids.push_back((unsigned)loc[edge_idx[e0 + e] & 0xffff] |
+                                     ((unsigned)loc[edge_idx[e0 + e] >> 16] << 16));
+            }
+        for (int f = 0; f < nf; ++f)
+            if (tri_of[f] == p) {
+                const uint2 ix = tri_idx[f0 + f];
+                S.tris.push_back(f);
+                S.tri_ids.push_back(make_uint2((unsigned)loc[ix.x & 0xffff] | ((unsigned)loc[ix.x >> 16] << 16),
+                                               (unsigned)loc[ix.y & 0xffff] | (ix.y & 0xffff0000u)));
+            }
+        P.nt = (int)S.tets.size() - P.t0; P.ne = (int)S.edges.size() - P.e0; P.nf = (int)S.tris.size() - P.f0;
+    }
+    return S;
+}
+
+// Threads of a part's block: one item (a tet or an edge) a thread as far as that goes, so
+// that a small part's edges run beside its tets
+int split_block(int items) {
+    return items <= 128 ? 128 : items <= 256 ? 256 : 512;
+}
+// Block size of a class whose envs are split, and its grid: as many clusters as the device
+// holds at once.
+int32_t configure_split(ffsrl_batch* b, ffsrl_batch::Class& c, int block, size_t dyn_budget) {
+    // (the block sizes an undivided class takes, rounded to the cluster kernels')
+    if (!kernel_f(b, block, 0, 0)) return fail(FFSRL_ERR_UNSUPPORTED, "ffsrl_batch: no kernel for block " + std::to_string(block));
+    block = split_block(block);
+    kern_f k = split_f(b, block);
+    cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_budget);
+    if (e == cudaSuccess && c.split > 8)
+        e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return cuda_fail(e, "ffsrl_batch: cluster kernel attribute");
+    c.block = block;
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = cluster_config(c, 1, at, nullptr);
+    int clusters = 0;
+    e = cudaOccupancyMaxActiveClusters(&clusters, (const void*)k, &cfg);
+    if (e != cudaSuccess || clusters <= 0) {
+        cudaGetLastError();
+        return fail(FFSRL_ERR_UNSUPPORTED, "ffsrl_batch: a cluster of " + std::to_string(c.split) + " blocks of " +
+                                               std::to_string(block) + " threads does not fit");
+    }
+    c.grid = std::min(c.members, clusters);
+    return FFSRL_OK;
+}
+
+// held[g]: how many clusters of g blocks, each with a block's whole shared-memory budget, the
+// device holds at once (0: none, or no size in use).
+std::vector<int> clusters_held(ffsrl_batch* b, size_t dyn_budget) {
+    std::vector<int> held(kMaxSplit + 1, 0);
+    held[1] = b->sm_count;
+    for (int g : kSplits) {
+        ffsrl_batch::Class c{};
+        c.members = INT_MAX;
+        c.smem = dyn_budget;
+        c.split = g;
+        if (configure_split(b, c, 512, dyn_budget) == FFSRL_OK) held[g] = c.grid;
+        else clear_error();
+    }
+    return held;
+}
+// Blocks per env (1: the env is not split).  An env's blocks are as many as bring a block's
+// cost to at most a limit that is the same for all envs; the limit is the one with the least
+// estimated time for the whole plan.  The estimate (cycles of one iteration, measured on the
+// liver constraint set): a block takes kFixed cycles for its barriers and per-vertex work
+// and so many per tet as its threads allow; a plan whose blocks the device holds all at once
+// takes as long as its costliest block, another one the SMs' mean load and part of a
+// costliest block at the end.
+std::vector<int> choose_split(const std::vector<int>& held, const std::vector<int64_t>& cost, const std::vector<int>& nt,
+                              const std::vector<int>& nv, bool fast) {
+    const size_t N = cost.size();
+    constexpr double kPerTet = 6.0;  // an env's cost is about six times its tets
+    const double kFixed1 = fast ? 3500.0 : 5000.0, kFixedCluster = fast ? 7000.0 : 9000.0;
+    auto blocks = [&](size_t e, double most) {
+        int g = 1;
+        for (int q : kSplits)
+            if (held[q] > 0 && (double)cost[e] / g > most && nt[e] >= q * kMinPartTets) g = q;
+        return g;
+    };
+    auto estimate = [&](double most) {
+        double longest = 0.0, load = 0.0, room = 0.0;
+        for (size_t e = 0; e < N; ++e) {
+            const int g = blocks(e, most);
+            const double tets = (double)cost[e] / kPerTet / g;
+            const int threads = g > 1 ? split_block((int)(1.2 * tets)) : default_block(nv[e], 0, N <= (size_t)held[1]);
+            const double rate = (threads >= 512 ? 12.5 : threads == 256 ? 27.0 : 50.0) * (fast ? 0.5 : 1.0);
+            const double t = (g > 1 ? kFixedCluster : kFixed1) + tets * rate;
+            const double per_sm = threads >= 512 ? 1.0 : (g > 1 ? 512.0 : 768.0) / threads;
+            longest = std::max(longest, t);
+            load += t / (held[g] * per_sm);
+            room += 1.0 / (held[g] * per_sm);
+        }
+        return room <= 1.0 ? longest : std::max(longest, load + 0.3 * longest);
+    };
+    double hi = 1.0;
+    for (int64_t c : cost) hi = std::max(hi, (double)c);
+    double best = hi, best_t = estimate(hi);
+    for (int k = 1; k <= 32; ++k) {
+        const double most = hi * std::pow((double)kMaxSplit, -k / 32.0), t = estimate(most);
+        if (t < 0.97 * best_t) { best = most; best_t = t; }
+    }
+    std::vector<int> g(N);
+    for (size_t e = 0; e < N; ++e) g[e] = blocks(e, best);
+    return g;
+}
+
+// Block size of a class: the instantiation, its shared-memory allowance and the grid
+// from the runtime's occupancy calculator.
 int32_t configure_class(ffsrl_batch* b, ffsrl_batch::Class& c, int block, size_t dyn_budget) {
+    if (c.split > 1) return configure_split(b, c, block, dyn_budget);
     if (b->precision == 64 || b->accum != FFSRL_ACC_FIXED) {
         // the float64 and accumulation-study builds have fewer block sizes: take the
         // nearest one at or above the request that exists
@@ -861,18 +1153,95 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
         edge_la.swap(n_edge_la);
     }
 
-    // ---- order each env's constraint records by a greedy vertex colouring ----
+    // ---- split envs over clusters of blocks (float32 fixed point without connectors): see
+    // choose_split; and an env whose state does not fit one block's shared memory is split
+    // until its parts fit (or, where they never do, keeps its storage mode).  No bit of the
+    // result depends on it. ----
+    b->env_cost.resize(N);
+    for (int e = 0; e < N; ++e) b->env_cost[e] = 4ll * env[e].nt + env[e].ne + env[e].nf + env[e].nv;
+    std::vector<int> split(N, 1), part_nv(N), part_nf(N), part_nx(N, 0);
+    std::vector<PartRec> part_rec;
+    std::vector<int> vmap, tet_pre, edge_pre;  // tet_pre: the record before the split's reordering
+    std::vector<unsigned> xch;
+    for (int e = 0; e < N; ++e) { part_nv[e] = env[e].nv; part_nf[e] = env[e].nf; }
+    if (precision == 32 && accum == FFSRL_ACC_FIXED && !conn) {
+        const std::vector<int> held = clusters_held(b, dyn_budget);
+        std::vector<int> nts(N), nvs(N);
+        for (int e = 0; e < N; ++e) { nts[e] = env[e].nt; nvs[e] = env[e].nv; }
+        const std::vector<int> want = choose_split(held, b->env_cost, nts, nvs, b->arith == FFSRL_ARITH_FAST);
+        tet_pre.resize(T);
+        edge_pre.resize(edge_idx.size());
+        std::iota(tet_pre.begin(), tet_pre.end(), 0);
+        std::iota(edge_pre.begin(), edge_pre.end(), 0);
+        auto reorder = [](auto& v, int o, const std::vector<int>& ids, int per = 1) {
+            if (v.empty()) return;
+            const auto c = std::decay_t<decltype(v)>(v.begin() + (size_t)per * o, v.begin() + (size_t)per * (o + ids.size()));
+            for (size_t i = 0; i < ids.size(); ++i)
+                for (int k = 0; k < per; ++k) v[(size_t)per * (o + i) + k] = c[(size_t)per * ids[i] + k];
+        };
+        std::unordered_map<int, Split> splits;  // by distinct env
+        for (int e = 0; e < N; ++e) {
+            EnvRec& r = env[e];
+            const int root = dup_of[e] >= 0 ? dup_of[e] : e;
+            if (root == e) {
+                int g = want[e];
+                if (plan_smem(b, 0, r.nv) > dyn_budget) g = std::max(g, 2);
+                for (; g > 1 && g <= kMaxSplit; ++g) {
+                    if (!held[g]) continue;
+                    Split S = split_env(g, r.nv, hm->vertex + 3ll * r.v0, tet_idx, r.t0, r.nt, edge_idx, r.e0, r.ne,
+                                        tri_idx, r.f0, r.nf);
+                    int nx = 0;
+                    for (const PartRec& P : S.parts) nx = std::max(nx, xch_words(P));
+                    if (plan_smem(b, 0, S.max_loc) + 8 + 4 * (size_t)nx > dyn_budget) continue;
+                    part_nx[e] = nx;
+                    r.p0 = (int)part_rec.size();
+                    for (PartRec P : S.parts) {
+                        P.map0 += (int)vmap.size();
+                        P.x0 += (int)xch.size();
+                        part_rec.push_back(P);
+                    }
+                    part_nv[e] = S.max_loc;
+                    part_nf[e] = 0;
+                    for (const PartRec& P : S.parts) part_nf[e] = std::max(part_nf[e], P.nf);
+                    vmap.insert(vmap.end(), S.vmap.begin(), S.vmap.end());
+                    xch.insert(xch.end(), S.xch.begin(), S.xch.end());
+                    split[e] = g;
+                    splits[e] = std::move(S);
+                    break;
+                }
+            }
+            const auto it = splits.find(root);
+            if (it == splits.end()) continue;
+            const Split& S = it->second;
+            split[e] = split[root]; part_nv[e] = part_nv[root]; part_nf[e] = part_nf[root]; part_nx[e] = part_nx[root]; r.p0 = env[root].p0;
+            reorder(tet_va, r.t0, S.tets); reorder(nh0, r.t0, S.tets); reorder(nh1, r.t0, S.tets);
+            reorder(nhd, r.t0, S.tets, 3); reorder(tet_vs, r.t0, S.tets); reorder(tet_ed, r.t0, S.tets);
+            reorder(tet_cls, r.t0, S.tets); reorder(tet_pre, r.t0, S.tets);
+            reorder(edge_la, r.e0, S.edges); reorder(edge_pre, r.e0, S.edges);
+            std::copy(S.tet_ids.begin(), S.tet_ids.end(), tet_idx.begin() + r.t0);
+            std::copy(S.edge_ids.begin(), S.edge_ids.end(), edge_idx.begin() + r.e0);
+            std::copy(S.tri_ids.begin(), S.tri_ids.end(), tri_idx.begin() + r.f0);
+        }
+    }
+
+    // ---- order each env's (each part's) constraint records by a greedy vertex colouring ----
     std::vector<int> tet_orig(T), edge_orig(edge_idx.size());
     {
         std::vector<uint64_t> used;
         std::vector<int> col;
-        for (int e = 0; e < N; ++e) {
-            const EnvRec& r = env[e];
+        for (int e = 0; e < N; ++e)
+        for (int p = 0; p < split[e]; ++p) {
+            EnvRec r = env[e];
             if (dup_of[e] >= 0) {
+                if (p > 0) break;
                 const EnvRec& src = env[dup_of[e]];
                 for (int j = 0; j < r.nt; ++j) tet_orig[r.t0 + j] = r.t0 + (tet_orig[src.t0 + j] - src.t0);
                 for (int j = 0; j < r.ne; ++j) edge_orig[r.e0 + j] = r.e0 + (edge_orig[src.e0 + j] - src.e0);
                 continue;
+            }
+            if (split[e] > 1) {
+                const PartRec& P = part_rec[r.p0 + p];
+                r.t0 += P.t0; r.nt = P.nt; r.e0 += P.e0; r.ne = P.ne; r.nv = P.n_loc;
             }
             used.assign(r.nv, 0);
             col.resize(std::max(r.nt, r.ne));
@@ -931,6 +1300,10 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
                 for (int k = 0; k < 3; ++k) nhd[3 * i + k] = c[3 * (size_t)tet_orig[i] + k];
         }
         permute(tet_vs, tet_orig); permute(tet_ed, tet_orig); permute(edge_idx, edge_orig); permute(edge_la, edge_orig);
+        if (!part_rec.empty()) {
+            for (int& t : tet_orig) t = tet_pre[t];
+            for (int& k : edge_orig) k = edge_pre[k];
+        }
     }
 
     // ---- compact fast-form records: the rest volume carries the volume constraint's
@@ -968,7 +1341,7 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
             auto eq = [](const auto& v, int o1, int o2, int n) {
                 return n == 0 || v.empty() || std::memcmp(&v[o1], &v[o2], sizeof(v[0]) * (size_t)n) == 0;
             };
-            return a.nv == c.nv && a.nt == c.nt && a.ne == c.ne && a.nf == c.nf &&
+            return a.nv == c.nv && a.nt == c.nt && a.ne == c.ne && a.nf == c.nf && a.p0 == c.p0 &&
                    eq(tet_idx, a.t0, c.t0, a.nt) && eq(tet_va, a.t0, c.t0, a.nt) && eq(nh0, a.t0, c.t0, a.nt) &&
                    eq(tet_ed2, a.t0, c.t0, a.nt) &&
                    eq(nhd, 3 * a.t0, 3 * c.t0, 3 * a.nt) &&
@@ -1019,7 +1392,7 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
     const int bands[] = {192, 384, 768, 1536, 3072, 65536};
     b->env_class.assign(N, -1);
     std::vector<std::vector<int>> members;
-    std::vector<int> keys;  // mode*16 + band
+    std::vector<int> keys;  // (cluster size, mode, band)
     auto mode_for = [&](int nv) {
         if (precision == 64) return plan_smem(b, 0, nv) <= dyn_budget ? 0 : 2;
         if (plan_smem(b, 0, nv) <= dyn_budget) return 0;
@@ -1029,43 +1402,69 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
     for (int e = 0; e < N; ++e) {
         int m = mode_for(env[e].nv);
         int band = 0;
-        while (env[e].nv > bands[band]) ++band;
-        int key = m * 16 + (m == 0 ? band : 0);
+        while (part_nv[e] > bands[band]) ++band;
+        int key = split[e] > 1 ? split[e] * 64 + m * 16 : m * 16 + (m == 0 ? band : 0);
         auto it = std::find(keys.begin(), keys.end(), key);
         int ci;
         if (it == keys.end()) { keys.push_back(key); members.emplace_back(); ci = (int)keys.size() - 1; }
         else ci = (int)(it - keys.begin());
         members[ci].push_back(e);
     }
-    // order classes by key for reproducible launch order
+    // the largest clusters are launched first, while they find enough SMs free side by side,
+    // then the class with the costliest block: its blocks would otherwise wait for those of
+    // the smaller classes, and then run alone
     std::vector<int> order(keys.size());
+    std::vector<int64_t> block_cost(keys.size(), 0);
+    for (size_t k = 0; k < keys.size(); ++k)
+        for (int e : members[k]) block_cost[k] = std::max(block_cost[k], b->env_cost[e] / split[e]);
     std::iota(order.begin(), order.end(), 0);
-    std::sort(order.begin(), order.end(), [&](int a, int c) { return keys[a] < keys[c]; });
+    std::sort(order.begin(), order.end(), [&](int a, int c) {
+        if (keys[a] / 64 != keys[c] / 64) return keys[a] > keys[c];
+        return block_cost[a] != block_cost[c] ? block_cost[a] > block_cost[c] : keys[a] < keys[c];
+    });
     size_t scratch_total = 0;
-    b->env_cost.resize(N);
-    for (int e = 0; e < N; ++e) b->env_cost[e] = 4ll * env[e].nt + env[e].ne + env[e].nf + env[e].nv;
     for (int oi : order) {
         auto& mem = members[oi];
         std::sort(mem.begin(), mem.end(), [&](int a, int c) {
             return b->env_cost[a] != b->env_cost[c] ? b->env_cost[a] > b->env_cost[c] : a < c;
         });
         ffsrl_batch::Class c{};
-        c.mode = keys[oi] / 16;
+        c.split = std::max(1, keys[oi] / 64);
+        c.mode = keys[oi] % 64 / 16;
         c.max_nv = 1;
-        for (int e : mem) c.max_nv = std::max(c.max_nv, env[e].nv);
-        c.smem = plan_smem(b, c.mode, c.max_nv);
+        for (int e : mem) {
+            c.max_nv = std::max(c.max_nv, part_nv[e]);
+            c.env_nv = std::max(c.env_nv, env[e].nv);
+        }
+        const int block_mode = c.split > 1 ? 0 : c.mode;  // a part always lives in shared memory
+        c.smem = plan_smem(b, block_mode, c.max_nv);
+        size_t xch_bytes = 0;
+        if (c.split > 1) {  // the exchange table, after the triangles
+            for (int e : mem) xch_bytes = std::max(xch_bytes, 4 * (size_t)part_nx[e]);
+            c.smem = (c.smem + 7) & ~(size_t)7;
+        }
         if (p->flags & FFSRL_COLLIDE) {
             // the contact scan reads every surface triangle in every iteration: keep the
             // env's triangles in shared memory when they fit
             int max_nf = 0;
-            for (int e : mem) max_nf = std::max(max_nf, env[e].nf);
+            for (int e : mem) max_nf = std::max(max_nf, part_nf[e]);
             const size_t with = ((c.smem + 7) & ~(size_t)7) + 8 * (size_t)max_nf;
-            if (max_nf > 0 && with <= dyn_budget) { c.tri_cap = max_nf; c.smem = with; }
+            if (max_nf > 0 && with + xch_bytes <= dyn_budget) { c.tri_cap = max_nf; c.smem = with; }
         }
-        c.scratch_stride = plan_scratch(b, c.mode, c.max_nv);
+        c.smem += xch_bytes;
+        c.scratch_stride = plan_scratch(b, block_mode, c.max_nv);
         c.scratch_stride = (c.scratch_stride + 255) & ~(size_t)255;
         c.members = (int)mem.size();
-        int want = block_override > 0 ? block_override : default_block(c.max_nv, c.mode);
+        int want = block_override > 0 ? block_override : default_block(c.max_nv, c.mode, N <= b->sm_count);
+        if (c.split > 1) {
+            int items = 0;
+            for (int e : mem)
+                for (int q = 0; q < c.split; ++q) {
+                    const PartRec& P = part_rec[env[e].p0 + q];
+                    items = std::max(items, ((P.nt + 31) & ~31) + P.ne);
+                }
+            if (block_override <= 0) want = split_block(items);
+        }
         if (int32_t st = configure_class(b, c, want, dyn_budget)) { free_batch(b); return st; }
         // scratch for the largest grid any block size can give (8 resident blocks per SM)
         c.scratch_offset = scratch_total;
@@ -1080,6 +1479,9 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
     if ((st = dalloc(b, &b->d_cnt0, (size_t)V)) || (st = upload(b->d_cnt0, cnt0)) ||
         (st = dalloc(b, &b->d_tet_orig, tet_orig.size())) || (st = upload(b->d_tet_orig, tet_orig)) ||
         (st = dalloc(b, &b->d_edge_orig, edge_orig.size())) || (st = upload(b->d_edge_orig, edge_orig)) ||
+        (st = dalloc(b, &b->d_part, part_rec.size())) || (st = upload(b->d_part, part_rec)) ||
+        (st = dalloc(b, &b->d_vmap, vmap.size())) || (st = upload(b->d_vmap, vmap)) ||
+        (st = dalloc(b, &b->d_xch, xch.size())) || (st = upload(b->d_xch, xch)) ||
         (st = dalloc(b, &b->d_env, N)) || (st = upload(b->d_env, env)) ||
         (st = dalloc(b, &b->d_tet_idx, tet_idx.size())) || (st = upload(b->d_tet_idx, tet_idx)) ||
         (st = dalloc(b, &b->d_tet_va, tet_va.size())) || (st = upload(b->d_tet_va, tet_va)) ||
@@ -1219,7 +1621,7 @@ extern "C" int32_t ffsrl_batch_class_info(const ffsrl_batch* b, int32_t cls, int
                                           int32_t* block, int32_t* num_envs) {
     if (!b || cls < 0 || cls >= (int)b->classes.size()) return fail(FFSRL_ERR_INVALID_ARGUMENT, "ffsrl_batch_class_info");
     const auto& c = b->classes[cls];
-    if (max_nv) *max_nv = c.max_nv;
+    if (max_nv) *max_nv = c.env_nv;
     if (mode) *mode = c.mode;
     if (block) *block = c.block;
     if (num_envs) *num_envs = c.work_count;

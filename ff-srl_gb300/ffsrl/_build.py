@@ -30,6 +30,8 @@ UNITS = {
     "plain.cu": ["-fmad=false"],
     "batched.cu": ["-prec-div=false", "-prec-sqrt=false"],
     "batched_ref.cu": ["-fmad=false"],
+    "batched_split.cu": ["-prec-div=false", "-prec-sqrt=false"],
+    "batched_split_ref.cu": ["-fmad=false"],
     "batched_study.cu": ["-fmad=false"],
     "render.cu": ["-fmad=false"],
     "instrument.cu": ["-fmad=false"],
