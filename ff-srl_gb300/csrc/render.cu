@@ -5,6 +5,7 @@
 // with IEEE division and square root the images and boxes equal the CPU restatement's
 // bit for bit whenever the summation order is the same (the fused paths).
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include "ffsrl_internal.h"
 #include "vecmath.cuh"
@@ -24,57 +25,62 @@ __device__ __forceinline__ int find_env(const int* __restrict__ node_offset, int
     return lo;
 }
 
-__device__ __forceinline__ void refit_node(const ffsrl_bvh& b, const float* __restrict__ pts,
+// A leaf's box from its triangles' vertices, and the packed copies of both
+__device__ __forceinline__ void refit_leaf(const ffsrl_bvh& b, const float* __restrict__ pts,
                                            const int* __restrict__ faces, int e, int n0, int t0, int base, int node) {
-    int left = b.left_node[n0 + node];
-    v3 lo, hi;
-    if (left < 0) {
-        lo = mk(1e6f, 1e6f, 1e6f);
-        hi = mk(-1e6f, -1e6f, -1e6f);
-        int first = b.first_tri_id[n0 + node];
-        int cnt = b.tri_count[n0 + node];
-        long long fofs = b.env_face_offset[e];
-        for (int k = 0; k < cnt; ++k) {
-            long long f = fofs + b.tri_id[t0 + first + k];
-            // the reference's refit may box another face than the one it traverses
-            // (bvh.py:66-74 against render.py:462-470); refit_source holds that face
-            const long long fb = b.refit_source ? (long long)b.refit_source[f] : f;
-            v3 pA = ld3(pts, faces[3 * fb]), pB = ld3(pts, faces[3 * fb + 1]), pC = ld3(pts, faces[3 * fb + 2]);
-            lo = vmin(pA, vmin(pB, vmin(pC, lo)));
-            hi = vmax(pA, vmax(pB, vmax(pC, hi)));
-            if (fb != f) pA = ld3(pts, faces[3 * f]), pB = ld3(pts, faces[3 * f + 1]), pC = ld3(pts, faces[3 * f + 2]);
-            if (b.tri_pos) {
-                float4* q = reinterpret_cast<float4*>(b.tri_pos) + 3 * (fofs + first + k);
-                q[0] = make_float4(pA.x, pA.y, pA.z, pB.x);
-                q[1] = make_float4(pB.y, pB.z, pC.x, pC.y);
-                q[2] = make_float4(pC.z, 0.0f, 0.0f, 0.0f);
-            }
+    v3 lo = mk(1e6f, 1e6f, 1e6f), hi = mk(-1e6f, -1e6f, -1e6f);
+    int first = b.first_tri_id[n0 + node];
+    int cnt = b.tri_count[n0 + node];
+    long long fofs = b.env_face_offset[e];
+    for (int k = 0; k < cnt; ++k) {
+        long long f = fofs + b.tri_id[t0 + first + k];
+        // the reference's refit may box another face than the one it traverses
+        // (bvh.py:66-74 against render.py:462-470); refit_source holds that face
+        const long long fb = b.refit_source ? (long long)b.refit_source[f] : f;
+        v3 pA = ld3(pts, faces[3 * fb]), pB = ld3(pts, faces[3 * fb + 1]), pC = ld3(pts, faces[3 * fb + 2]);
+        lo = vmin(pA, vmin(pB, vmin(pC, lo)));
+        hi = vmax(pA, vmax(pB, vmax(pC, hi)));
+        if (fb != f) pA = ld3(pts, faces[3 * f]), pB = ld3(pts, faces[3 * f + 1]), pC = ld3(pts, faces[3 * f + 2]);
+        if (b.tri_pos) {
+            float4* q = reinterpret_cast<float4*>(b.tri_pos) + 3 * (fofs + first + k);
+            q[0] = make_float4(pA.x, pA.y, pA.z, pB.x);
+            q[1] = make_float4(pB.y, pB.z, pC.x, pC.y);
+            q[2] = make_float4(pC.z, 0.0f, 0.0f, 0.0f);
         }
-        if (b.node_box) {
-            float4* nb = reinterpret_cast<float4*>(b.node_box) + 2ll * (base + node);
-            nb[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(-1));
-            nb[1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(first * 256 + (cnt < 255 ? cnt : 255)));
-        }
-    } else {
-        v3 l0 = ld3(b.aabb_min, base + left), h0 = ld3(b.aabb_max, base + left);
-        v3 l1 = ld3(b.aabb_min, base + left + 1), h1 = ld3(b.aabb_max, base + left + 1);
-        lo = vmin(l0, l1);
-        hi = vmax(h0, h1);
-        if (b.node_box) {
-            // the traversal's child order: the axis along which the children's centres lie
-            // farthest apart (bits 0-1) and whether the right child's centre is the higher
-            // one (bit 2)
-            const v3 d = (l1 + h1) - (l0 + h0);
-            const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-            const int axis = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
-            const float da = axis == 0 ? d.x : (axis == 1 ? d.y : d.z);
-            float4* nb = reinterpret_cast<float4*>(b.node_box) + 2ll * (base + node);
-            nb[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(left));
-            nb[1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(axis | (da > 0.0f ? 4 : 0)));
-        }
+    }
+    if (b.node_box) {
+        float4* nb = reinterpret_cast<float4*>(b.node_box) + 2ll * (base + node);
+        nb[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(-1));
+        nb[1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(first * 256 + (cnt < 255 ? cnt : 255)));
     }
     st3(b.aabb_min, base + node, lo);
     st3(b.aabb_max, base + node, hi);
+}
+
+// An inner node's box from its children's (l0, h0 the left one's), and the packed copy
+__device__ __forceinline__ void refit_inner(const ffsrl_bvh& b, int base, int node, int left, v3 l0, v3 h0, v3 l1,
+                                            v3 h1, v3& lo, v3& hi) {
+    lo = vmin(l0, l1);
+    hi = vmax(h0, h1);
+    if (b.node_box) {
+        // the traversal's child order: the axis along which the children's centres lie
+        // farthest apart (bits 0-1) and whether the right child's centre is the higher
+        // one (bit 2)
+        const v3 d = (l1 + h1) - (l0 + h0);
+        const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+        const int axis = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
+        const float da = axis == 0 ? d.x : (axis == 1 ? d.y : d.z);
+        float4* nb = reinterpret_cast<float4*>(b.node_box) + 2ll * (base + node);
+        nb[0] = make_float4(lo.x, lo.y, lo.z, __int_as_float(left));
+        nb[1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(axis | (da > 0.0f ? 4 : 0)));
+    }
+    st3(b.aabb_min, base + node, lo);
+    st3(b.aabb_max, base + node, hi);
+}
+__device__ __forceinline__ void refit_inner_global(const ffsrl_bvh& b, int base, int node, int left) {
+    v3 lo, hi;
+    refit_inner(b, base, node, left, ld3(b.aabb_min, base + left), ld3(b.aabb_max, base + left),
+                ld3(b.aabb_min, base + left + 1), ld3(b.aabb_max, base + left + 1), lo, hi);
 }
 
 // refitBVHLevel (bvh.py:30-104): every env node at `level`
@@ -87,24 +93,178 @@ __global__ void k_refit_level(ffsrl_bvh b, const float* __restrict__ pts, const 
     int node = tid - b.env_node_offset[e];
     if (node >= b.topo_node_offset[topo + 1] - n0) return;
     if (b.level[n0 + node] != level) return;
-    refit_node(b, pts, faces, e, n0, b.topo_tri_offset[topo], b.env_node_offset[e], node);
+    const int left = b.left_node[n0 + node];
+    if (left < 0) refit_leaf(b, pts, faces, e, n0, b.topo_tri_offset[topo], b.env_node_offset[e], node);
+    else refit_inner_global(b, b.env_node_offset[e], node, left);
 }
 
-// One block per env (or per listed env): levels deepest first, nodes of a level in parallel.
-__global__ void k_refit_fused(ffsrl_bvh b, const float* __restrict__ pts, const int* __restrict__ faces,
-                              const int* __restrict__ ids) {
-    int e = ids ? ids[blockIdx.x] : blockIdx.x;
+// The fused refit runs in two launches: every leaf of every env (or listed env) at once, one
+// thread a node, then the inner nodes of an env by one block.  (One block that did an env's
+// leaves and levels in turn waited for global memory some five times a level: with cold caches
+// 72 us for one env of 2,180 faces, 101 for 8 of 1,400 to 4,400, 112 for 256; the two launches
+// take 34, 51 and 94.)
+__global__ void __launch_bounds__(256) k_refit_leaves(ffsrl_bvh b, const float* __restrict__ pts,
+                                                      const int* __restrict__ faces, const int* __restrict__ ids,
+                                                      int chunks) {
+    const int k = blockIdx.x / chunks, e = ids ? ids[k] : k;
     if (e < 0 || e >= b.num_envs) return;
-    int topo = b.env_topology[e];
-    int n0 = b.topo_node_offset[topo], t0 = b.topo_tri_offset[topo];
-    int base = b.env_node_offset[e];
-    int lo = b.topo_level_offset[topo];
-    int groups = b.topo_max_level[topo] + 1;
-    for (int g = 0; g < groups; ++g) {
-        int s0 = b.level_start[lo + g], s1 = b.level_start[lo + g + 1];
-        for (int k = s0 + threadIdx.x; k < s1; k += blockDim.x) refit_node(b, pts, faces, e, n0, t0, base, b.level_node[k]);
+    const int topo = b.env_topology[e], n0 = b.topo_node_offset[topo];
+    const int nn = b.topo_node_offset[topo + 1] - n0, t0 = b.topo_tri_offset[topo], base = b.env_node_offset[e];
+    for (int node = (blockIdx.x % chunks) * blockDim.x + threadIdx.x; node < nn; node += chunks * blockDim.x)
+        if (b.left_node[n0 + node] < 0) refit_leaf(b, pts, faces, e, n0, t0, base, node);
+}
+
+// Shared memory of the climb: per node its left child and its parent (2 bytes each), per inner
+// node its box (24 bytes) and a bit for the first child to arrive
+__host__ __device__ inline size_t climb_bytes(int nn) {
+    return 24 * (size_t)(nn / 2 + 1) + 4 * (size_t)(nn / 64 + 1) + 4 * (size_t)nn;
+}
+
+// Inner nodes of one env per block.  The build numbers the two children of a node 2s + 1 and
+// 2s + 2, so pair s stands for an inner node.  A thread takes a pair: two leaves make their
+// parent's box at once, a leaf beside an inner node hands its box over, two inner nodes are
+// left to others; a thread with a box climbs on for as long as it is the second of a node's
+// two children to arrive.  The climb stays in shared memory (a level costs an atomic there
+// instead of a barrier and trips to L2), reads the leaves' boxes coalesced and one pair
+// ahead, and leaves what goes to global memory to a last pass over all pairs.  The same box
+// whichever child comes second: the left child's box is always the first operand.  An env
+// whose tree is numbered in another way or does not fit the block's shared memory is refitted
+// level by level from global memory.
+__global__ void __launch_bounds__(1024) k_refit_climb(ffsrl_bvh b, const int* __restrict__ ids, int smem_bytes) {
+    extern __shared__ float climb_smem[];
+    __shared__ int s_bad;
+    const int e = ids ? ids[blockIdx.x] : blockIdx.x;
+    if (e < 0 || e >= b.num_envs) return;
+    const int topo = b.env_topology[e], n0 = b.topo_node_offset[topo];
+    const int nn = b.topo_node_offset[topo + 1] - n0, base = b.env_node_offset[e], step = blockDim.x;
+    constexpr unsigned short kNone = 0xffffu;
+    float* box = climb_smem;                                              // box[6 s]: the node whose children are pair s
+    unsigned* arrived = reinterpret_cast<unsigned*>(box + 6 * (nn / 2 + 1));  // bit s
+    unsigned short* left = reinterpret_cast<unsigned short*>(arrived + nn / 64 + 1);  // kNone: a leaf
+    unsigned short* parent = left + nn;
+    const bool fits = nn < 65535 && (nn & 1) && climb_bytes(nn) <= (size_t)smem_bytes;
+    if (fits) {
+        if (threadIdx.x == 0) s_bad = 0;
+        for (int i = threadIdx.x; i < nn; i += step) parent[i] = kNone;
+        for (int i = threadIdx.x; i < nn / 64 + 1; i += step) arrived[i] = 0u;
+        __syncthreads();
+        for (int i0 = threadIdx.x; i0 < nn; i0 += 4 * step) {
+            int l[4];  // four loads in flight
+            for (int k = 0; k < 4; ++k) l[k] = i0 + k * step < nn ? b.left_node[n0 + i0 + k * step] : -1;
+            for (int k = 0; k < 4; ++k) {
+                const int i = i0 + k * step;
+                if (i >= nn) break;
+                left[i] = l[k] < 0 ? kNone : (unsigned short)l[k];
+                if (l[k] < 0) continue;
+                if (!(l[k] & 1) || l[k] + 1 >= nn || i >= l[k]) s_bad = 1;
+                else parent[l[k]] = parent[l[k] + 1] = (unsigned short)i;
+            }
+        }
+        __syncthreads();
+        // a tree: every pair has a parent, and the one that names it
+        for (int s = threadIdx.x; s < nn / 2; s += step) {
+            const unsigned short p = parent[2 * s + 1];
+            if (p == kNone || left[p] != 2 * s + 1) s_bad = 1;
+        }
+        for (int i = threadIdx.x; i < nn; i += step)  // no two nodes with the same children
+            if (left[i] != kNone && !s_bad && parent[left[i]] != i) s_bad = 1;
         __syncthreads();
     }
+    if (fits && !s_bad) {
+        struct Pair { v3 l0, h0, l1, h1; };
+        auto load_pair = [&](int s) {  // (of an inner child nothing is used)
+            Pair q;
+            const long long g = base + 2ll * s + 1;
+            q.l0 = ld3(b.aabb_min, g); q.l1 = ld3(b.aabb_min, g + 1);
+            q.h0 = ld3(b.aabb_max, g); q.h1 = ld3(b.aabb_max, g + 1);
+            return q;
+        };
+        auto get = [&](int s, v3& lo, v3& hi) {
+            const volatile float* q = box + 6 * s;
+            lo = mk(q[0], q[1], q[2]);
+            hi = mk(q[3], q[4], q[5]);
+        };
+        auto put = [&](int s, v3 lo, v3 hi) {
+            volatile float* q = box + 6 * s;
+            q[0] = lo.x; q[1] = lo.y; q[2] = lo.z; q[3] = hi.x; q[4] = hi.y; q[5] = hi.z;
+        };
+        const int pairs = nn / 2;
+        Pair nx;
+        if ((int)threadIdx.x < pairs) nx = load_pair(threadIdx.x);
+        for (int s0 = threadIdx.x; s0 < pairs; s0 += step) {
+            const Pair q = nx;
+            if (s0 + step < pairs) nx = load_pair(s0 + step);
+            const bool leaf0 = left[2 * s0 + 1] == kNone, leaf1 = left[2 * s0 + 2] == kNone;
+            if (!leaf0 && !leaf1) continue;
+            int s = s0;         // the pair this thread's box belongs to
+            bool right = !leaf0;  // ... and which of the two it is
+            v3 lo = leaf0 ? q.l0 : q.l1, hi = leaf0 ? q.h0 : q.h1;
+            bool done = leaf0 && leaf1;  // the pair's node has both its boxes
+            if (done) {
+                lo = vmin(q.l0, q.l1);
+                hi = vmax(q.h0, q.h1);
+            } else {
+                put(s, lo, hi);  // a leaf's box waits in its parent's place
+            }
+            for (;;) {
+                if (!done) {
+                    const unsigned bit = 1u << (s & 31);
+                    __threadfence_block();
+                    if (!(atomicOr(arrived + (s >> 5), bit) & bit)) break;
+                    __threadfence_block();
+                    const int sib = 2 * s + (right ? 1 : 2);
+                    v3 sl, sh;
+                    get(left[sib] == kNone ? s : left[sib] >> 1, sl, sh);
+                    lo = right ? vmin(sl, lo) : vmin(lo, sl);
+                    hi = right ? vmax(sh, hi) : vmax(hi, sh);
+                }
+                put(s, lo, hi);
+                const int p = parent[2 * s + 1];  // the node this box is of
+                if (p == 0) break;
+                s = (p - 1) >> 1;
+                right = !(p & 1);
+                done = false;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < pairs) nx = load_pair(threadIdx.x);
+        for (int s = threadIdx.x; s < pairs; s += step) {
+            Pair q = nx;
+            if (s + step < pairs) nx = load_pair(s + step);
+            if (left[2 * s + 1] != kNone) get(left[2 * s + 1] >> 1, q.l0, q.h0);
+            if (left[2 * s + 2] != kNone) get(left[2 * s + 2] >> 1, q.l1, q.h1);
+            v3 lo, hi;
+            refit_inner(b, base, parent[2 * s + 1], 2 * s + 1, q.l0, q.h0, q.l1, q.h1, lo, hi);
+        }
+        return;
+    }
+    const int first = b.topo_level_offset[topo], groups = b.topo_max_level[topo] + 1;
+    for (int g = 0; g < groups; ++g) {
+        const int s0 = b.level_start[first + g], s1 = b.level_start[first + g + 1];
+        for (int k = s0 + threadIdx.x; k < s1; k += blockDim.x) {
+            const int node = b.level_node[k], left = b.left_node[n0 + node];
+            if (left >= 0) refit_inner_global(b, base, node, left);
+        }
+        __syncthreads();
+    }
+}
+
+// Both launches for n envs (ids null: all)
+int32_t refit_fused(const ffsrl_bvh& b, const float* pts, const int32_t* faces, const int32_t* ids, int n, cudaStream_t s) {
+    int dev = 0, sms = 0, most = 0;
+    FFSRL_CUDA_TRY(cudaGetDevice(&dev));
+    FFSRL_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    FFSRL_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const int mean = b.total_env_nodes / b.num_envs;
+    const int chunks = std::max(1, std::min(mean / 256 + 1, 64));
+    k_refit_leaves<<<(unsigned)((long long)chunks * n), 256, 0, s>>>(b, pts, faces, ids, chunks);
+    // up to an env per SM a block has the SM's shared memory (trees to 14,300 nodes) and 1,024
+    // threads; with more, two blocks share it (7,100 nodes)
+    const bool few = n <= sms;
+    const int smem = (few ? most : most / 2) - 1024 - 256;
+    FFSRL_CUDA_TRY(cudaFuncSetAttribute(k_refit_climb, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_refit_climb<<<n, few ? 1024 : 512, smem, s>>>(b, ids, smem);
+    return FFSRL_OK;
 }
 
 __global__ void k_zero3(float* p, int n) {
@@ -622,7 +782,7 @@ extern "C" int32_t ffsrl_bvh_refit_fused(const ffsrl_bvh* b, const float* pts, c
     if (int32_t st = check_bvh(b)) return st;
     if (!pts || !faces || !b->level_node || !b->level_start || !b->topo_level_offset)
         return fail(FFSRL_ERR_INVALID_ARGUMENT, "ffsrl_bvh_refit_fused: needs level grouping arrays");
-    k_refit_fused<<<b->num_envs, 256, 0, (cudaStream_t)stream>>>(*b, pts, faces, nullptr);
+    if (int32_t st = refit_fused(*b, pts, faces, nullptr, b->num_envs, (cudaStream_t)stream)) return st;
     FFSRL_LAUNCH_CHECK("ffsrl_bvh_refit_fused");
     return FFSRL_OK;
 }
@@ -666,7 +826,7 @@ extern "C" int32_t ffsrl_bvh_refit_fused_envs(const ffsrl_bvh* b, const float* p
     if (n < 0 || (n > 0 && (!pts || !faces || !env_ids || !b->level_node || !b->level_start || !b->topo_level_offset)))
         return fail(FFSRL_ERR_INVALID_ARGUMENT, "ffsrl_bvh_refit_fused_envs");
     if (n == 0) return FFSRL_OK;
-    k_refit_fused<<<n, 256, 0, (cudaStream_t)stream>>>(*b, pts, faces, env_ids);
+    if (int32_t st = refit_fused(*b, pts, faces, env_ids, n, (cudaStream_t)stream)) return st;
     FFSRL_LAUNCH_CHECK("ffsrl_bvh_refit_fused_envs");
     return FFSRL_OK;
 }
