@@ -592,14 +592,14 @@ __device__ __forceinline__ v3 texel(const ffsrl_render& r, const int* ob, int lf
     return (1.0f - ay) * lower + ay * upper;
 }
 
-__device__ __forceinline__ Shade trace(const ffsrl_render& r, const EnvView& ev, int e, v3 ro, float4 q, int x, int y,
-                                       int W, int H) {
+__device__ __forceinline__ v3 ray_dir(const ffsrl_render& r, float4 q, int x, int y, int W, int H) {
     float sx = 2.0f * float(x) / float(W) - 1.0f;
     float sy = 2.0f * float(y) / float(H) - 1.0f;
-    v3 rd = normalize(quat_rotate(q, mk(sx * r.camera_tan * r.camera_aspect, sy * r.camera_tan, -1.0f)));
-    float t = 0.0f;
-    v3 p = mk(0.0f, 0.0f, 0.0f);
-    int tri = query(ev, r.vis_point, r.vis_face, ro, rd, t, p, r.error_flag);
+    return normalize(quat_rotate(q, mk(sx * r.camera_tan * r.camera_aspect, sy * r.camera_tan, -1.0f)));
+}
+
+// colour and depth of a ray's hit: global face `tri` (-1: none) at distance t, point p
+__device__ __forceinline__ Shade shade(const ffsrl_render& r, const EnvView& ev, int e, int tri, float t, v3 p) {
     Shade s;
     s.color = mk(0.0f, 0.0f, 0.0f);
     s.depth = 0.0f;
@@ -648,6 +648,15 @@ __device__ __forceinline__ Shade trace(const ffsrl_render& r, const EnvView& ev,
     return s;
 }
 
+__device__ __forceinline__ Shade trace(const ffsrl_render& r, const EnvView& ev, int e, v3 ro, float4 q, int x, int y,
+                                       int W, int H) {
+    const v3 rd = ray_dir(r, q, x, y, W, H);
+    float t = 0.0f;
+    v3 p = mk(0.0f, 0.0f, 0.0f);
+    const int tri = query(ev, r.vis_point, r.vis_face, ro, rd, t, p, r.error_flag);
+    return shade(r, ev, e, tri, t, p);
+}
+
 // drawSimBVHKernelManyEnvs (render.py:276-409): one thread per ray, into scratch
 __global__ void k_draw(ffsrl_render r, ffsrl_bvh b) {
     const int W = 2 * r.resolution, H = 2 * r.resolution;
@@ -686,35 +695,10 @@ __global__ void k_downsample(ffsrl_render r) {
     if (r.depth) r.depth[tid] = d / nsq;
 }
 
-// One thread per ray; the four rays of a pixel sit in consecutive lanes and are summed
-// by shuffles in downsample_kernel's order ((r00 + r01) + r10) + r11, then divided by 4.
-// A block covers an 8x8 pixel tile of one env so neighbouring rays share BVH nodes in L1,
-// and a warp's rays cover a compact 4x2-pixel patch (3% faster than a row of 8 pixels:
-// closer rays take more of the same nodes).
-__global__ void __launch_bounds__(256) k_rays(ffsrl_render r, ffsrl_bvh b, const int* __restrict__ ids, int n_ids) {
-    const int R = r.resolution, W = 2 * R, H = 2 * R;
-    const int tiles_x = (R + 7) / 8;
-    const int tiles = tiles_x * ((R + 7) / 8);
-    const int k = blockIdx.x / tiles;
-    const int e = ids ? (k < n_ids ? ids[k] : r.num_envs) : k;
-    const int tile = blockIdx.x % tiles;
-    const int pix = threadIdx.x >> 2, q = threadIdx.x & 3;
-    // a warp's eight pixels form a 4x2 patch; the tile's eight warps form 2x4 patches
-    const int wp = pix >> 3, j = pix & 7;
-    const int px = (tile % tiles_x) * 8 + (wp & 1) * 4 + (j & 3);
-    const int py = (tile / tiles_x) * 8 + (wp >> 1) * 2 + (j >> 2);
-    const bool valid = e >= 0 && e < r.num_envs && px < R && py < R;
-    Shade s;
-    s.color = mk(0.0f, 0.0f, 0.0f);
-    s.depth = 0.0f;
-    if (valid) {
-        const int cam = r.num_cameras > 1 ? e : 0;
-        const v3 ro = ld3(r.camera_pos, cam);
-        const float4 qr = reinterpret_cast<const float4*>(r.camera_rot)[cam];
-        const EnvView ev = env_view(b, e);
-        const int et = (2 * py + (q >> 1)) * W + 2 * px + (q & 1);  // ray index as in downsample_kernel
-        s = trace(r, ev, e, ro, qr, et % W, H - et / W, W, H);
-    }
+// The four rays of a pixel sit in consecutive lanes: summed by shuffles in
+// downsample_kernel's order ((r00 + r01) + r10) + r11, then divided by 4.
+__device__ __forceinline__ void store_pixel(const ffsrl_render& r, const Shade& s, bool valid, int e, int px, int py) {
+    const int R = r.resolution, q = threadIdx.x & 3;
     float cx = s.color.x, cy = s.color.y, cz = s.color.z, d = s.depth;
     float ax[3], ay[3], az[3], ad[3];
 #pragma unroll
@@ -733,6 +717,387 @@ __global__ void __launch_bounds__(256) k_rays(ffsrl_render r, ffsrl_bvh b, const
         if (r.color) st3(r.color, o, mk(c.x / nsq, c.y / nsq, c.z / nsq));
         if (r.depth) r.depth[o] = dd / nsq;
     }
+}
+
+// ---- bundles of rays -----------------------------------------------------------------
+// Ray directions (not normalised) as d0 + x dx + y dy over the ray indices
+struct Camera { v3 d0, dx, dy; };
+__device__ __forceinline__ Camera make_camera(const ffsrl_render& r, float4 q, int W, int H) {
+    const float tx = r.camera_tan * r.camera_aspect, ty = r.camera_tan;
+    Camera c;
+    c.d0 = quat_rotate(q, mk(-tx, -ty, -1.0f));
+    c.dx = quat_rotate(q, mk(2.0f * tx / float(W), 0.0f, 0.0f));
+    c.dy = quat_rotate(q, mk(0.0f, 2.0f * ty / float(H), 0.0f));
+    return c;
+}
+// The four corners of a rectangle of w x h pixels' rays from pixel (px, py), widened by a
+// quarter of the ray spacing on each side: far more than rounding moves a ray's direction
+// (some 3e-7), so every ray of the rectangle lies between the corners
+struct Corners { v3 d[4]; };
+__device__ __forceinline__ Corners make_corners(const Camera& c, int px, int py, int w, int h, int H) {
+    const float x0 = 2.0f * px - 0.25f, x1 = 2.0f * (px + w) - 0.75f;
+    const float y0 = H - (2.0f * (py + h) - 0.75f), y1 = H - (2.0f * py - 0.25f);
+    const v3 a = c.d0 + x0 * c.dx, b = c.d0 + x1 * c.dx;
+    Corners k;
+    k.d[0] = a + y0 * c.dy; k.d[1] = b + y0 * c.dy; k.d[2] = b + y1 * c.dy; k.d[3] = a + y1 * c.dy;
+    return k;
+}
+// The planes through the camera between them, normals inward; outside() leaves a relative
+// 2e-6 on top, as the slab test sees a box's edges with that much rounding.  (A zero or
+// non-finite normal excludes nothing.)
+struct Bundle { v3 n[4]; };
+__device__ __forceinline__ Bundle make_bundle(const Corners& k) {
+    const v3 c = (k.d[0] + k.d[2]) + (k.d[1] + k.d[3]);
+    Bundle b;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const v3 n = cross(k.d[i], k.d[(i + 1) & 3]);
+        const float m = fabsf(n.x) + fabsf(n.y) + fabsf(n.z);
+        const float f = __fdividef(dot(n, c) < 0.0f ? -1.0f : 1.0f, m);
+        b.n[i] = m > 0.0f ? n * f : mk(0.0f, 0.0f, 0.0f);
+    }
+    return b;
+}
+
+__device__ __forceinline__ float fdot(v3 a, v3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
+__device__ __forceinline__ v3 fcross(v3 a, v3 b) {
+    return mk(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
+}
+__device__ __forceinline__ float sum1(v3 a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
+
+// Whether a ray between the corners can pass the triangle test: its determinant and the
+// numerators of u and v are linear in the direction, so where the determinant has one sign
+// at all corners, and u, v or 1 - u - v the wrong one, by more than the test's own rounding
+// (some 1e-6 of the vectors' lengths; 1e-5 here), no ray does.
+__device__ __forceinline__ bool may_hit(const Corners& k, v3 ab, v3 ac, v3 tv, v3 qv) {
+    const v3 N = fcross(ac, ab), U = fcross(ac, tv);
+    float dlo = 3.4e38f, dhi = -3.4e38f, ulo = dlo, uhi = dhi, vlo = dlo, vhi = dhi, wlo = dlo, whi = dhi, len = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float d = fdot(k.d[i], N), u = fdot(k.d[i], U), v = fdot(k.d[i], qv), w = (d - u) - v;
+        dlo = fminf(dlo, d); dhi = fmaxf(dhi, d);
+        ulo = fminf(ulo, u); uhi = fmaxf(uhi, u);
+        vlo = fminf(vlo, v); vhi = fmaxf(vhi, v);
+        wlo = fminf(wlo, w); whi = fmaxf(whi, w);
+        len = fmaxf(len, sum1(k.d[i]));
+    }
+    const float a = sum1(ab), c = sum1(ac), t = sum1(tv);
+    const float gu = 1e-5f * len * t * c, gv = 1e-5f * len * t * a, gd = 1e-5f * len * a * c, gw = gu + gv + gd;
+    if (dlo > gd) return !(uhi < -gu || vhi < -gv || whi < -gw);
+    if (dhi < -gd) return !(ulo > gu || vlo > gv || wlo > gw);
+    return true;
+}
+
+// whether the box [lo, hi], relative to the camera, lies outside one of the planes
+__device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
+    const v3 c = mk(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
+    const v3 h = mk(0.5f * (hi.x - lo.x), 0.5f * (hi.y - lo.y), 0.5f * (hi.z - lo.z));
+    const float g = 2e-6f * ((fabsf(c.x) + fabsf(c.y)) + (fabsf(c.z) + h.x) + (h.y + h.z));
+    bool out = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const v3 n = b.n[k];
+        float s = fmaf(fabsf(n.x), h.x, fmaf(fabsf(n.y), h.y, fmaf(fabsf(n.z), h.z, g)));
+        s = fmaf(n.x, c.x, fmaf(n.y, c.y, fmaf(n.z, c.z, s)));
+        out |= s < 0.0f;
+    }
+    return out;
+}
+
+// Ray-cast by tiles of T x T pixels, 256 threads each.  What a thread per ray spends its time
+// on is the walk down the tree, which neighbouring rays share.  Here a block finds the leaves
+// that its tile's rays can reach, all its threads testing a level of the tree at a time
+// against the tile's bundle; it prepares their triangles in shared memory (what the triangle
+// test computes from the camera and the triangle alone, the faces towards the camera first);
+// then each warp takes patches of 4 x 2 pixels (32 rays), keeps the listed triangles its
+// patch's rays can reach, a triangle a lane, and tests them one after another, all lanes the
+// same triangle.  A tile with more triangles than the list holds is done in quarters.
+// 256 envs of 500-20,000 tets at 128 x 128: a thread per ray took 1,224 us and 1,900
+// instructions a warp of 32 rays with two thirds of its lanes busy, the tiles 730; 8 textured
+// envs at 512 x 512: 540 and 275 us.  What bounds it now is issue, 65% of it, and on one env
+// the chain of loads, tests and shading of the tile with the most triangles (45 us).
+//
+// The hit is the traversal's: of the triangles whose test succeeds, the nearest, the first
+// in the reference's order among equals.  The traversal reaches a triangle if the ray's slab
+// test enters its leaf's box (it then enters the boxes above, as rounding is monotone) and
+// no hit before it is nearer than that entry, so the nearest one's leaf is put to the slab
+// test at the end.  In the rare case that the test fails, or puts the entry behind another
+// hit (two triangles hit in a box's corner, where the one that is kept hangs on the order of
+// the traversal), the ray is traversed.  So is a ray along a coordinate plane, and every ray
+// of a 4 x 4 tile that still has too many triangles, or of a tree deeper than kSteps levels
+// below the ones tested first.
+constexpr int kCand = 448;      // triangles of a tile, 64 bytes of shared memory each
+constexpr int kFront = 768;     // nodes of a level
+constexpr int kSteps = 40;
+constexpr int kList = 160;      // triangles a warp keeps for its four patches
+// Levels tested at once at the start.  Large images (T 16): at most 255 nodes, one a thread.
+// Small ones wait for each step more than for its work: at most 2,047 nodes, eight a thread.
+template <int T> struct FirstLevel { static constexpr int value = T == 16 ? 7 : 10; };
+
+// The traversal of one ray, kept out of line: few rays take it
+struct Hit { int tri; float t; v3 p; };
+__device__ __noinline__ Hit traverse(const ffsrl_render* r, const ffsrl_bvh* b, int e, v3 ro, v3 rd) {
+    Hit h;
+    h.t = 0.0f;
+    h.p = mk(0.0f, 0.0f, 0.0f);
+    h.tri = query(env_view(*b, e), r->vis_point, r->vis_face, ro, rd, h.t, h.p, r->error_flag);
+    return h;
+}
+
+template <int T>
+__global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_render r, const __grid_constant__ ffsrl_bvh b,
+                                                 const int* __restrict__ ids, int n_ids) {
+    __shared__ float4 s_tri[4 * kCand];  // (ab, ac, tvec, qvec, ac.qvec, leaf, place in the leaf, distance)
+    __shared__ unsigned short s_list[T == 16 ? 8 : 1][kList];
+    __shared__ int s_front[2][kFront];
+    __shared__ int s_leaf[kCand];
+    __shared__ int s_n[3], s_leaves, s_over, s_nf, s_nb;
+    __shared__ int s_todo[8][3];  // tiles still to do: x, y, size
+    const int R = r.resolution, W = 2 * R, H = 2 * R;
+    const int tiles_x = (R + T - 1) / T, tiles = tiles_x * tiles_x;
+    const int k = blockIdx.x / tiles;
+    const int e = ids ? (k < n_ids ? ids[k] : r.num_envs) : k;
+    if (e < 0 || e >= r.num_envs) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cam = r.num_cameras > 1 ? e : 0;
+    const v3 ro = ld3(r.camera_pos, cam);
+    const float4 qr = reinterpret_cast<const float4*>(r.camera_rot)[cam];
+    const EnvView ev = env_view(b, e);
+    const Camera cm = make_camera(r, qr, W, H);
+    const bool packed = ev.box && ev.tpos;
+    int todo = 0;  // tiles in s_todo, the same for every thread
+    int tx = ((blockIdx.x % tiles) % tiles_x) * T, ty = ((blockIdx.x % tiles) / tiles_x) * T, size = T;
+    for (;;) {
+        if (tid < 3) s_n[tid] = 0;
+        if (tid == 0) { s_leaves = 0; s_over = 0; s_nf = 0; s_nb = 0; }
+        __syncthreads();
+        if (packed) {
+            const Bundle F = make_bundle(make_corners(cm, tx, ty, size, size, H));
+            auto visit = [&](int node, int* count, int* front, bool expand) {
+                if ((unsigned)node >= (unsigned)ev.nn) { s_over = 1; return; }
+                const float4 a = __ldg(ev.box + 2 * node), c = __ldg(ev.box + 2 * node + 1);
+                const int left = __float_as_int(a.w);
+                if (left != -1 && !expand) return;
+                if (outside(F, mk(a.x, a.y, a.z) - ro, mk(c.x, c.y, c.z) - ro)) return;
+                if (left == -1) {
+                    const int q = atomicAdd(&s_leaves, 1);
+                    if (q < kCand) s_leaf[q] = node;
+                } else {
+                    const int q = atomicAdd(count, 2);
+                    if (left >= 0 && left + 1 < ev.nn && q + 1 < kFront) {
+                        front[q] = left;
+                        front[q + 1] = left + 1;
+                    } else {
+                        s_over = 1;
+                    }
+                }
+            };
+            // the nodes of the first level and the leaves above them, from the level lists (deepest
+            // level first), or the root
+            if (b.level_node && b.level_start && b.topo_level_offset) {
+                const int topo = b.env_topology[e], lo = b.topo_level_offset[topo], deepest = b.topo_max_level[topo];
+                const int g = max(0, deepest - FirstLevel<T>::value);
+                const int s0 = b.level_start[lo + g], s1 = b.level_start[lo + g + 1], s2 = b.level_start[lo + deepest + 1];
+                for (int i0 = s0 + tid; i0 < s2; i0 += 1024) {
+                    int node[4];  // four loads in flight
+                    for (int m = 0; m < 4; ++m) node[m] = i0 + 256 * m < s2 ? b.level_node[i0 + 256 * m] : -1;
+                    for (int m = 0; m < 4; ++m)
+                        if (i0 + 256 * m < s2) visit(node[m], &s_n[0], s_front[0], i0 + 256 * m < s1);
+                }
+            } else if (tid == 0) {
+                visit(0, &s_n[0], s_front[0], true);
+            }
+            __syncthreads();
+            // step j takes the s_n[j % 3] nodes of s_front[j & 1]; every thread sees the same
+            // count, as step j + 1 is the next to change it
+            int step = 0;
+            for (;; ++step) {
+                const int n = min(s_n[step % 3], kFront);
+                if (n == 0 || step == kSteps) break;
+                if (tid == 0) s_n[(step + 2) % 3] = 0;
+                for (int i = tid; i < n; i += 256)
+                    visit(s_front[step & 1][i], &s_n[(step + 1) % 3], s_front[(step + 1) & 1], true);
+                __syncthreads();
+            }
+            if (step == kSteps && tid == 0) s_over = 1;
+            const int leaves = min(s_leaves, kCand);
+            for (int i = tid; i < leaves; i += 256) {
+                const int node = s_leaf[i];
+                const float4 a = __ldg(ev.box + 2 * node), c = __ldg(ev.box + 2 * node + 1);
+                const int fc = __float_as_int(c.w), first = fc >> 8;
+                int cnt = fc & 255;
+                if (cnt == 255) cnt = ev.count[node];
+                // distance of the box, a little less: no ray hits in it nearer than that
+                const v3 lo = mk(a.x, a.y, a.z) - ro, hi = mk(c.x, c.y, c.z) - ro;
+                const v3 gap = mk(fmaxf(fmaxf(lo.x, -hi.x), 0.0f), fmaxf(fmaxf(lo.y, -hi.y), 0.0f), fmaxf(fmaxf(lo.z, -hi.z), 0.0f));
+                const float near = length(gap) * 0.9999f;
+                for (int m = 0; m < cnt; ++m) {
+                    const float4* q = ev.tpos + 3ll * (first + m);
+                    const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
+                    const v3 A = mk(q0.x, q0.y, q0.z);
+                    const v3 ab = mk(q0.w, q1.x, q1.y) - A, ac = mk(q1.z, q1.w, q2.x) - A, tv = ro - A, qv = cross(tv, ab);
+                    const float tn = dot(ac, qv);
+                    const int at = tn > 0.0f ? atomicAdd(&s_nf, 1) : kCand - 1 - atomicAdd(&s_nb, 1);
+                    if ((unsigned)at >= (unsigned)kCand) continue;  // too many: counted below
+                    s_tri[4 * at] = make_float4(ab.x, ab.y, ab.z, ac.x);
+                    s_tri[4 * at + 1] = make_float4(ac.y, ac.z, tv.x, tv.y);
+                    s_tri[4 * at + 2] = make_float4(tv.z, qv.x, qv.y, qv.z);
+                    s_tri[4 * at + 3] = make_float4(tn, __int_as_float(node), __int_as_float(m), near);
+                }
+            }
+        }
+        __syncthreads();
+        int nf = s_nf, nb = s_nb;  // triangles facing the camera, and others
+        const bool listed = packed && !s_over && s_leaves <= kCand && nf + nb <= kCand;
+        if (packed && !listed && size > 4) {
+            // the quarters instead (at most 3 + 4 tiles wait at a time)
+            size >>= 1;
+            if (tid < 4) {
+                s_todo[todo + tid][0] = tx + (tid & 1) * size;
+                s_todo[todo + tid][1] = ty + (tid >> 1) * size;
+                s_todo[todo + tid][2] = size;
+            }
+            todo += 4;
+        } else {
+            // the triangles of the list from which a warp's rays can hit, by lane: whether triangle
+            // c is one of them for the rays between corners k
+            auto reach = [&](const Corners& k, int c) {
+                const float4 A = s_tri[4 * c], B = s_tri[4 * c + 1], C = s_tri[4 * c + 2];
+                return may_hit(k, mk(A.x, A.y, A.z), mk(A.w, B.x, B.y), mk(B.z, B.w, C.x), mk(C.y, C.z, C.w));
+            };
+            // a warp's patches: four of 4 x 2 pixels in a region of 8 x 4 (tiles of 16), or one.
+            // The region's triangles are picked from the tile's first, a patch's from those.
+            const bool four = T == 16 && size == 16;
+            const int rx = tx + (size == 4 ? 0 : (warp & 1) * (four ? 8 : 4));
+            const int ry = ty + (size == 4 ? warp * 2 : (warp >> 1) * (four ? 4 : 2));
+            bool own = false;  // the warp's list is s_list, or the tile's
+            if (four && listed && nf + nb > 32) {
+                const Corners K = make_corners(cm, rx, ry, 8, 4, H);
+                int n = 0, f = 0;
+                for (int side = 0; side < 2; ++side) {
+                    const int c0 = side ? kCand - nb : 0, c1 = side ? kCand : nf;
+                    for (int cb = c0; cb < c1; cb += 32) {
+                        const bool in = cb + lane < c1 && reach(K, cb + lane);
+                        const unsigned mask = __ballot_sync(0xffffffffu, in);
+                        const int at = n + __popc(mask & ((1u << lane) - 1u));
+                        if (in && at < kList) s_list[T == 16 ? warp : 0][at] = (unsigned short)(cb + lane);
+                        n += __popc(mask);
+                    }
+                    if (!side) f = n;
+                }
+                if (n <= kList) { own = true; nf = f; nb = n - f; }
+                __syncwarp();
+            }
+            for (int patch = 0; patch < (four ? 4 : 1) && (size > 4 || warp < 2); ++patch) {
+                const int pw = rx + (patch & 1) * 4, ph = ry + (patch >> 1) * 2;
+                const int j = lane >> 2, q = lane & 3;
+                const int px = pw + (j & 3), py = ph + (j >> 2);
+                const bool valid = px < R && py < R;
+                Shade s;
+                s.color = mk(0.0f, 0.0f, 0.0f);
+                s.depth = 0.0f;
+                if (!listed || nf + nb > 0) {
+                    const v3 rd = ray_dir(r, qr, 2 * px + (q & 1), H - (2 * py + (q >> 1)), W, H);  // ray as in downsample_kernel
+                    // a ray along a coordinate plane: its slab test has no finite distances, so a
+                    // leaf may be entered and a box above it not
+                    bool walk = valid && (!listed || rd.x == 0.0f || rd.y == 0.0f || rd.z == 0.0f);
+                    Hit hit;
+                    hit.tri = -1; hit.t = 0.0f; hit.p = mk(0.0f, 0.0f, 0.0f);
+                    if (listed) {
+                        const Corners K = make_corners(cm, pw, ph, 4, 2, H);
+                        float tMin = valid && !walk ? 1e6f : 0.0f;  // (a lane at 0 hits nothing)
+                        float second = 1e6f;  // the nearest hit but for the best one
+                        int best = -1;
+                        // moller_trumbore on a prepared triangle, in two parts.  First the numerators
+                        // against the determinant, by more than rounding: a division only for
+                        // the triangles a ray is in, or nearly
+                        auto near_in = [&](int c, float& det, float& nu, float& nv) {
+                            const float4 A = s_tri[4 * c], B = s_tri[4 * c + 1], C = s_tri[4 * c + 2];
+                            const v3 pvec = cross(rd, mk(A.w, B.x, B.y));
+                            det = dot(mk(A.x, A.y, A.z), pvec);
+                            nu = dot(mk(B.z, B.w, C.x), pvec);
+                            nv = dot(rd, mk(C.y, C.z, C.w));
+                            const float ad = fabsf(det), su = det < 0.0f ? -nu : nu, sv = det < 0.0f ? -nv : nv;
+                            return !(ad < 0.0001f || su < -1e-30f || sv < -1e-30f || su > 1.00001f * ad || su + sv > 1.00002f * ad);
+                        };
+                        auto test = [&](int c, float det, float nu, float nv) {
+                            const float4 D = s_tri[4 * c + 3];
+                            const float invDet = 1.0f / det;
+                            const float u = nu * invDet;
+                            if (u < 0.0f || u > 1.0f) return;
+                            const float v = nv * invDet;
+                            if (v < 0.0f || u + v > 1.0f) return;
+                            const float t = D.x * invDet;
+                            if (!(t > 0.0f)) return;
+                            if (t > tMin) { second = fminf(second, t); return; }
+                            second = tMin;
+                            if (t == tMin) {  // the traversal keeps the first of equals in the reference's order
+                                if (best < 0) return;
+                                const float4 E = s_tri[4 * best + 3];
+                                const int f0 = ev.first[__float_as_int(D.y)], f1 = ev.first[__float_as_int(E.y)];
+                                if (!(f0 > f1 || (f0 == f1 && __float_as_int(D.z) < __float_as_int(E.z)))) return;
+                            }
+                            tMin = t;
+                            best = c;
+                        };
+                        for (int side = 0; side < 2; ++side) {
+                            const int c0 = !side ? 0 : own ? nf : kCand - nb, c1 = c0 + (side ? nb : nf);
+                            for (int cb = c0; cb < c1; cb += 32) {
+                                // what lies behind every ray's hit so far is left out
+                                const float far = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(tMin)));
+                                int c = cb + lane;
+                                bool in = c < c1;
+                                if (in) {
+                                    if (own) c = s_list[T == 16 ? warp : 0][c];
+                                    in = s_tri[4 * c + 3].w <= far && reach(K, c);
+                                }
+                                unsigned mask = __ballot_sync(0xffffffffu, in);
+                                while (mask) {  // two at a time: a patch full of triangles waits for each in turn
+                                    const int l0 = __ffs(mask) - 1;
+                                    mask &= mask - 1;
+                                    const int l1 = mask ? __ffs(mask) - 1 : l0;
+                                    const int ca = __shfl_sync(0xffffffffu, c, l0), cb2 = __shfl_sync(0xffffffffu, c, l1);
+                                    float da, ua, va, db, ub, vb;
+                                    const bool ia = near_in(ca, da, ua, va), ib = near_in(cb2, db, ub, vb) && mask;
+                                    mask &= mask - 1;
+                                    if (ia) test(ca, da, ua, va);
+                                    if (ib) test(cb2, db, ub, vb);
+                                }
+                            }
+                        }
+                        if (best >= 0) {
+                            const float4 D = s_tri[4 * best + 3];
+                            const int leaf = __float_as_int(D.y);
+                            const float4 a = __ldg(ev.box + 2 * leaf), c = __ldg(ev.box + 2 * leaf + 1);
+                            float tn;
+                            if (slab(ro, rd, mk(a.x, a.y, a.z), mk(c.x, c.y, c.z), tn) && (tn <= tMin || tn < second)) {
+                                hit.t = tMin;
+                                hit.p = ro + tMin * rd;
+                                hit.tri = (int)(ev.fofs + ev.tri[ev.first[leaf] + __float_as_int(D.z)]);
+                            } else {
+                                walk = true;
+                            }
+                        }
+                    }
+                    if (walk) hit = traverse(&r, &b, e, ro, rd);
+                    if (valid) s = shade(r, ev, e, hit.tri, hit.t, hit.p);
+                }
+                store_pixel(r, s, valid, e, px, py);
+            }
+        }
+        if (todo == 0) return;
+        __syncthreads();
+        --todo;
+        tx = s_todo[todo][0]; ty = s_todo[todo][1]; size = s_todo[todo][2];
+    }
+}
+
+// Tiles of 16 pixels share the walk among 32 patches; tiles of 8, four times as many, where
+// those of 16 would give an SM fewer than seven
+void launch_rays(const ffsrl_render& r, const ffsrl_bvh& b, const int32_t* ids, int n, cudaStream_t s) {
+    auto tiles = [&](int t) { return ((long long)(r.resolution + t - 1) / t) * ((r.resolution + t - 1) / t) * n; };
+    if (tiles(16) >= 1024) k_rays<16><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n);
+    else k_rays<8><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
 }
 
 int32_t check_bvh(const ffsrl_bvh* b) {
@@ -814,8 +1179,7 @@ extern "C" int32_t ffsrl_render_fused(const ffsrl_render* r, const ffsrl_bvh* b,
     const int P = r->num_vis_points;
     k_normal_gather<<<grid_for(P, 256), 256, 0, s>>>(r->vis_point, r->vis_face, r->point_face_start, r->point_face,
                                                      r->vertex_normal, P);
-    const int tiles = ((r->resolution + 7) / 8) * ((r->resolution + 7) / 8);
-    k_rays<<<(unsigned)((long long)tiles * r->num_envs), 256, 0, s>>>(*r, *b, nullptr, 0);
+    launch_rays(*r, *b, nullptr, r->num_envs, s);
     FFSRL_LAUNCH_CHECK("ffsrl_render_fused");
     return FFSRL_OK;
 }
@@ -841,8 +1205,7 @@ extern "C" int32_t ffsrl_render_fused_envs(const ffsrl_render* r, const ffsrl_bv
     cudaStream_t s = (cudaStream_t)stream;
     k_normal_gather_envs<<<n, 256, 0, s>>>(r->vis_point, r->vis_face, r->point_face_start, r->point_face,
                                            r->vertex_normal, r->env_point_start, env_ids, r->num_envs);
-    const int tiles = ((r->resolution + 7) / 8) * ((r->resolution + 7) / 8);
-    k_rays<<<(unsigned)((long long)tiles * n), 256, 0, s>>>(*r, *b, env_ids, n);
+    launch_rays(*r, *b, env_ids, n, s);
     FFSRL_LAUNCH_CHECK("ffsrl_render_fused_envs");
     return FFSRL_OK;
 }
