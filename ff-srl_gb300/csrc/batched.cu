@@ -762,7 +762,12 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
                 const float* f = hm->tetrahedron_dm_inv + 9ll * t;
                 nhd[3 * t] = make_float4(f[0], f[1], f[2], f[3]);
                 nhd[3 * t + 1] = make_float4(f[4], f[5], f[6], f[7]);
-                nhd[3 * t + 2] = make_float4(f[8], 0.0f, 0.0f, 0.0f);
+                const float v0 = tet_va[t].x;
+                nhd[3 * t + 2] = make_float4(f[8], p->volume_compliance / p->dt / p->dt / v0,
+                                             p->deviatoric_compliance / p->dt / p->dt / v0,
+                                             v0);
+                const unsigned off = kInactive;
+                if (tet_va[t].y != 1.0f) std::memcpy(&nhd[3 * t + 2].w, &off, sizeof(off));
             }
             if (nh && !ex) {
                 // M = D D^T and det D of the stored D = Dm^-1 (row-major), in double
