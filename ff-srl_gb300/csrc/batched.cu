@@ -246,9 +246,11 @@ template <> int32_t launch_class<float>(ffsrl_batch* b, const ffsrl_batch::Class
     if (c.split > 1) {
         cudaLaunchAttribute at[1];
         cudaLaunchConfig_t cfg = cluster_config(c, grid, at, s);
-        FFSRL_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, (const Dev<float>)D, work, nwork, counter, nsteps, (unsigned char*)nullptr,
-                                          0ll, c.max_nv, 0, c.tri_cap));
-        return FFSRL_OK;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k, (const Dev<float>)D, work, nwork, counter, nsteps,
+                                                 (unsigned char*)nullptr, 0ll, c.max_nv, 0, c.tri_cap);
+        if (e == cudaSuccess) return FFSRL_OK;
+        cudaGetLastError();  // (the launch has recorded it, too)
+        return cuda_fail(e, "ffsrl_batch: cluster step kernel");
     }
     k<<<grid, c.block, c.smem, s>>>(D, work, nwork, counter, nsteps, scratch + c.scratch_offset,
                                     (long long)c.scratch_stride, c.max_nv, c.prefetch == 1 ? 1 : 0, c.tri_cap);
