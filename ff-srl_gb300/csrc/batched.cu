@@ -146,17 +146,19 @@ void free_batch(ffsrl_batch* b) {
     delete b;
 }
 
-// Threads of an undivided env's block.  `few`: the plan has at most one env per SM, so that a
-// block has its SM to itself and more warps shorten it; with more envs, smaller blocks share
-// an SM better (2048 mixed envs, fast arithmetic: 17.1 ms with 256 threads up to 1,024
-// vertices, 18.2 with 512).  768 threads are the most whose registers hold the tet loop: of
+// Threads of an undivided env's block.  `few`: the plan has at most few_envs envs, so that
+// small blocks would not fill the SMs together and more warps shorten each (512 and 1024 mixed
+// envs, reference: 10.1 and 20.0 ms with 512 threads up to 1,024 vertices, 11.2 and 23.3 with
+// 256; 512, fast: 5.5 and 5.7); with more envs, smaller blocks share an SM better (2048 mixed
+// envs, reference: 38.9 ms with 256, 40.1 with 512; 1024, fast: 8.9 and 9.2).  768 threads are the most whose registers hold the tet loop: of
 // 80 envs of 10k-19k tets a step took 8.96 ms (reference) and 4.20 ms (fast), against 9.69
 // and 4.74 with 1,024 threads, which spill.  With the sums in global scratch (mode 1) the
 // 46,640-tet ellipsoid took 37.1 ms with 512 threads, 42.9 with 1,024.
+int few_envs(const ffsrl_batch* b) { return (b->arith == FFSRL_ARITH_FAST ? 4 : 7) * b->sm_count; }
 int default_block(int max_nv, int mode, bool few) {
     if (mode == 2) return 256;
     if (max_nv > 2560) return mode == 1 ? 512 : 768;
-    if (max_nv > 1024 || few) return 512;
+    if (max_nv > 1024 || (few && max_nv > 64)) return 512;
     return max_nv <= 256 ? 128 : 256;
 }
 
@@ -527,16 +529,18 @@ Split split_env(int G, int nv, const float* x, const std::vector<uint2>& tet_idx
 }
 
 // Threads of a part's block: one item (a tet or an edge) a thread as far as that goes, so
-// that a small part's edges run beside its tets
+// that a small part's edges run beside its tets; a large part takes the most warps that hold
+// the tet loop in registers (16 ellipsoids of 46,640 tets, fast: 2.27 ms with 768 threads, 2.39
+// with 512; one, reference: 2.07 and 2.26)
 int split_block(int items) {
-    return items <= 128 ? 128 : items <= 256 ? 256 : 512;
+    return items <= 128 ? 128 : items <= 256 ? 256 : items <= 1024 ? 512 : 768;
 }
 // Block size of a class whose envs are split, and its grid: as many clusters as the device
 // holds at once.
 int32_t configure_split(ffsrl_batch* b, ffsrl_batch::Class& c, int block, size_t dyn_budget) {
     // (the block sizes an undivided class takes, rounded to the cluster kernels')
     if (!kernel_f(b, block, 0, 0)) return fail(FFSRL_ERR_UNSUPPORTED, "ffsrl_batch: no kernel for block " + std::to_string(block));
-    block = split_block(block);
+    block = block > 640 ? 768 : block > 256 ? 512 : block;
     kern_f k = split_f(b, block);
     cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_budget);
     if (e == cudaSuccess && c.split > 8)
@@ -572,46 +576,63 @@ std::vector<int> clusters_held(ffsrl_batch* b, size_t dyn_budget) {
     return held;
 }
 // Blocks per env (1: the env is not split).  An env's blocks are as many as bring a block's
-// cost to at most a limit that is the same for all envs; the limit is the one with the least
-// estimated time for the whole plan.  The estimate (cycles of one iteration, measured on the
-// liver constraint set): a block takes kFixed cycles for its barriers and per-vertex work
-// and so many per tet as its threads allow; a plan whose blocks the device holds all at once
-// takes as long as its costliest block, another one the SMs' mean load and part of a
-// costliest block at the end.
+// cost to at most a limit that is the same for all envs; the limit is the one whose plan ends
+// first when its blocks are handed to the SMs in the order they are launched, one a SM.  A
+// block's time (cycles of an iteration, measured on the liver constraint set, without contact):
+// so many for vertex passes and barriers, so many per round of its threads over the tets, at
+// least one round.  With more envs than few_envs the blocks even out
+// by themselves and none is split.
 std::vector<int> choose_split(const std::vector<int>& held, const std::vector<int64_t>& cost, const std::vector<int>& nt,
-                              const std::vector<int>& nv, bool fast) {
+                              const std::vector<int>& nv, bool fast, bool nh) {
     const size_t N = cost.size();
+    std::vector<int> g(N, 1);
     constexpr double kPerTet = 6.0;  // an env's cost is about six times its tets
-    const double kFixed1 = fast ? 3500.0 : 5000.0, kFixedCluster = fast ? 7000.0 : 9000.0;
-    auto blocks = [&](size_t e, double most) {
-        int g = 1;
-        for (int q : kSplits)
-            if (held[q] > 0 && (double)cost[e] / g > most && nt[e] >= q * kMinPartTets) g = q;
-        return g;
+    const double base1 = fast ? 3000.0 : 4500.0, base_cluster = fast ? 5000.0 : 6500.0;
+    auto round = [&](int threads) {
+        const double ref = threads == 768 ? 8750.0 : threads == 512 ? 6750.0 : threads == 256 ? 4800.0 : 4200.0;
+        return ref * (fast ? (threads == 768 ? 0.49 : 0.53) : 1.0) * (nh ? 1.0 : 0.65);
     };
-    auto estimate = [&](double most) {
-        double longest = 0.0, load = 0.0, room = 0.0;
+    auto blocks = [&](size_t e, double most) {
+        int n = 1;
+        for (int q : kSplits)
+            if (held[q] > 0 && (double)cost[e] / n > most && nt[e] >= q * kMinPartTets) n = q;
+        return n;
+    };
+    std::vector<size_t> order(N);
+    std::vector<double> time(N), free(held[1]);
+    auto ends = [&](double most) {
         for (size_t e = 0; e < N; ++e) {
-            const int g = blocks(e, most);
-            const double tets = (double)cost[e] / kPerTet / g;
-            const int threads = g > 1 ? split_block((int)(1.2 * tets)) : default_block(nv[e], 0, N <= (size_t)held[1]);
-            const double rate = (threads >= 512 ? 12.5 : threads == 256 ? 27.0 : 50.0) * (fast ? 0.5 : 1.0);
-            const double t = (g > 1 ? kFixedCluster : kFixed1) + tets * rate;
-            const double per_sm = threads >= 512 ? 1.0 : (g > 1 ? 512.0 : 768.0) / threads;
-            longest = std::max(longest, t);
-            load += t / (held[g] * per_sm);
-            room += 1.0 / (held[g] * per_sm);
+            g[e] = blocks(e, most);
+            const double tets = (double)cost[e] / kPerTet / g[e];
+            const int threads = g[e] > 1 ? split_block((int)(1.2 * tets)) : default_block(nv[e], 0, true);
+            time[e] = (g[e] > 1 ? base_cluster : base1) + std::max(1.0, tets / threads) * round(threads);
         }
-        return room <= 1.0 ? longest : std::max(longest, load + 0.3 * longest);
+        std::iota(order.begin(), order.end(), (size_t)0);
+        std::sort(order.begin(), order.end(), [&](size_t a, size_t c) {
+            return g[a] != g[c] ? g[a] > g[c] : time[a] != time[c] ? time[a] > time[c] : a < c;
+        });
+        std::fill(free.begin(), free.end(), 0.0);
+        double last = 0.0;
+        for (size_t e : order) {  // the group of g[e] SMs that is free first
+            const int n = g[e];
+            int best = 0;
+            double start = INFINITY;
+            for (int k = 0; k < held[n]; ++k) {
+                const double f = *std::max_element(free.begin() + k * n, free.begin() + (k + 1) * n);
+                if (f < start) { start = f; best = k; }
+            }
+            std::fill(free.begin() + best * n, free.begin() + (best + 1) * n, start + time[e]);
+            last = std::max(last, start + time[e]);
+        }
+        return last;
     };
     double hi = 1.0;
     for (int64_t c : cost) hi = std::max(hi, (double)c);
-    double best = hi, best_t = estimate(hi);
+    double best = hi, best_t = ends(hi);
     for (int k = 1; k <= 32; ++k) {
-        const double most = hi * std::pow((double)kMaxSplit, -k / 32.0), t = estimate(most);
-        if (t < 0.97 * best_t) { best = most; best_t = t; }
+        const double most = hi * std::pow((double)kMaxSplit, -k / 32.0), t = ends(most);
+        if (t < 0.98 * best_t) { best = most; best_t = t; }
     }
-    std::vector<int> g(N);
     for (size_t e = 0; e < N; ++e) g[e] = blocks(e, best);
     return g;
 }
@@ -1175,7 +1196,8 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
         const std::vector<int> held = clusters_held(b, dyn_budget);
         std::vector<int> nts(N), nvs(N);
         for (int e = 0; e < N; ++e) { nts[e] = env[e].nt; nvs[e] = env[e].nv; }
-        const std::vector<int> want = choose_split(held, b->env_cost, nts, nvs, b->arith == FFSRL_ARITH_FAST);
+        const std::vector<int> want = N <= few_envs(b) ? choose_split(held, b->env_cost, nts, nvs, !ex, nh)
+                                                      : std::vector<int>(N, 1);
         tet_pre.resize(T);
         edge_pre.resize(edge_idx.size());
         std::iota(tet_pre.begin(), tet_pre.end(), 0);
@@ -1462,7 +1484,7 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
         c.scratch_stride = plan_scratch(b, block_mode, c.max_nv);
         c.scratch_stride = (c.scratch_stride + 255) & ~(size_t)255;
         c.members = (int)mem.size();
-        int want = block_override > 0 ? block_override : default_block(c.max_nv, c.mode, N <= b->sm_count);
+        int want = block_override > 0 ? block_override : default_block(c.max_nv, c.mode, N <= few_envs(b));
         if (c.split > 1) {
             int items = 0;
             for (int e : mem)
