@@ -338,14 +338,36 @@ __global__ void k_collide(const float* xp, float* cdp, const int* __restrict__ t
         open = hole[f] == 1;
         a = tri[3 * f]; b = tri[3 * f + 1]; c = tri[3 * f + 2];
     }
+    // each capsule's box (its segment lies within a radius of base..tip), and its reach
+    v3 clo[3], chi[3];
+    for (int i = 0; i < 3; ++i) {
+        const long long k = 4ll * env + i;
+        const v3 p = ld3(base, k), q = ld3(tip, k);
+        const float mag = fmaxf(fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(p.z), fabsf(q.x))), fmaxf(fabsf(q.y), fabsf(q.z)));
+        const float m = 2.0f * radius[k] + 1e-4f * (1.0f + mag);
+        clo[i] = mk(fminf(p.x, q.x) - m, fminf(p.y, q.y) - m, fminf(p.z, q.z) - m);
+        chi[i] = mk(fmaxf(p.x, q.x) + m, fmaxf(p.y, q.y) + m, fmaxf(p.z, q.z) + m);
+    }
     wait_for_previous();
     if (open) return;
     v3 pA = ldw3(xp, a), pB = ldw3(xp, b), pC = ldw3(xp, c);
+    // A response needs a point of the capsule's segment within its radius of a point of the
+    // triangle, so there is none where the boxes are apart (the margin, 1e-4 of the
+    // coordinates, is far above their rounding).  A triangle without one adds nothing.  NaN
+    // coordinates are not apart from anything.
+    const v3 lo = vmin(pA, vmin(pB, pC)), hi = vmax(pA, vmax(pB, pC));
+    const float sum = ((pA.x + pA.y) + (pA.z + pB.x)) + ((pB.y + pB.z) + (pC.x + pC.y)) + pC.z;
+    unsigned near = 0;
+    for (int i = 0; i < 3; ++i)
+        if (isnan(sum) || !(lo.x > chi[i].x || lo.y > chi[i].y || lo.z > chi[i].z || hi.x < clo[i].x || hi.y < clo[i].y || hi.z < clo[i].z))
+            near |= 1u << i;
+    if (!near) return;
     v3 centre = (pA + pB + pC) * 0.3333f;
     v3 nrm = normalize(cross(pB - pA, pC - pA));
     v3 tA = mk(0.0f, 0.0f, 0.0f), tB = tA, tC = tA;
     float tl = 0.0f;
     for (int i = 0; i < 3; ++i) {
+        if (!((near >> i) & 1u)) continue;
         long long k = 4ll * env + i;
         v3 rA = mk(0.0f, 0.0f, 0.0f), rB = rA, rC = rA;
         capsule_response(ld3(tip, k), ld3(base, k), radius[k], nrm, centre, pA, pB, pC, ks, rA, rB, rC);
@@ -353,6 +375,7 @@ __global__ void k_collide(const float* xp, float* cdp, const int* __restrict__ t
         tl = tl + length(rA) + length(rB) + length(rC);
     }
     if (tl > 0.0f) atomicAdd(in_collision + env, 1);
+    if (!(tl > 0.0f) && !isnan(tl)) return;  // every response is zero
     if (inv_mass[a] > 0.0f) atomic_add3_pair(cdp, a, tA);
     if (inv_mass[b] > 0.0f) atomic_add3_pair(cdp, b, tB);
     if (inv_mass[c] > 0.0f) atomic_add3_pair(cdp, c, tC);
