@@ -235,6 +235,7 @@ Dev<float> make_dev_f(ffsrl_batch* b) {
     D.vol_c = p.volume_compliance; D.dev_c = p.deviatoric_compliance;
     D.a_dist = (float)((double)p.distance_compliance / ((double)p.dt * (double)p.dt));
     D.a_vol = (float)((double)p.volume_compliance_xpbd / ((double)p.dt * (double)p.dt));
+    D.nzero = 0x8000000080000000ull;
     return D;
 }
 
@@ -281,7 +282,7 @@ template <> int32_t launch_class<double>(ffsrl_batch* b, const ffsrl_batch::Clas
     D.tet_ed = F.tet_ed; D.tet_ed2 = nullptr; D.compact = 0; D.fold = F.fold;
     D.iterations = F.iterations; D.dt = F.dt; D.gx = F.gx; D.gy = F.gy; D.gz = F.gz; D.damping = F.damping;
     D.ground = F.ground; D.ks_distance = F.ks_distance; D.ks_volume = F.ks_volume; D.ks_contact = F.ks_contact;
-    D.ks_drag = F.ks_drag; D.vol_c = F.vol_c; D.dev_c = F.dev_c; D.a_dist = F.a_dist; D.a_vol = F.a_vol;
+    D.nzero = F.nzero; D.ks_drag = F.ks_drag; D.vol_c = F.vol_c; D.dev_c = F.dev_c; D.a_dist = F.a_dist; D.a_vol = F.a_vol;
     int grid = std::min(c.grid, nwork);
     if (grid <= 0) return FFSRL_OK;
     k<<<grid, c.block, c.smem, s>>>(D, work, nwork, counter, nsteps, scratch + c.scratch_offset,
