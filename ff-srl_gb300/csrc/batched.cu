@@ -146,19 +146,23 @@ void free_batch(ffsrl_batch* b) {
     delete b;
 }
 
-// Threads of an undivided env's block.  `few`: the plan has at most few_envs envs, so that
-// small blocks would not fill the SMs together and more warps shorten each (512 and 1024 mixed
-// envs, reference: 10.1 and 20.0 ms with 512 threads up to 1,024 vertices, 11.2 and 23.3 with
-// 256; 512, fast: 5.5 and 5.7); with more envs, smaller blocks share an SM better (2048 mixed
-// envs, reference: 38.9 ms with 256, 40.1 with 512; 1024, fast: 8.9 and 9.2).  768 threads are the most whose registers hold the tet loop: of
-// 80 envs of 10k-19k tets a step took 8.96 ms (reference) and 4.20 ms (fast), against 9.69
-// and 4.74 with 1,024 threads, which spill.  With the sums in global scratch (mode 1) the
-// 46,640-tet ellipsoid took 37.1 ms with 512 threads, 42.9 with 1,024.
-int few_envs(const ffsrl_batch* b) { return (b->arith == FFSRL_ARITH_FAST ? 4 : 7) * b->sm_count; }
+// Threads of an undivided env's block.  768 are the most whose registers hold the tet loop
+// (1,024 spill), and one such block fills an SM as 512 threads do, whose registers come to
+// as many: 152 envs of 1,448 vertices took 2.04 ms (reference) and 1.16 ms (fast) a step
+// with 768, 2.26 and 1.30 with 512; of 304 vertices there is nothing between them.  `few`:
+// the plan has at most few_envs envs, so that smaller blocks, three to an SM, would not fill
+// the SMs; with more envs they do, up to the size at which their shared memory leaves no
+// room for three (912 envs of 1,448 vertices: 11.9 and 6.5 ms with 256, 12.1 and 6.9 with
+// 768; of 2,171: 34.0 and 11.3 against 22.8 and 10.0).  few_envs, mixed pools of 500-20,000
+// tets: 700 and 900 envs, fast, 6.3 and 8.1 ms as few, 7.2 and 8.5 as many, 1,100 as fast
+// either way; 800, reference, 12.3 and 14.0, 1,200 17.8 either way.  With the sums in global
+// scratch (mode 1) the 46,640-tet ellipsoid took 37.1 ms with 512 threads, 42.9 with 1,024.
+int few_envs(const ffsrl_batch* b) { return (b->arith == FFSRL_ARITH_FAST ? 6 : 7) * b->sm_count; }
 int default_block(int max_nv, int mode, bool few) {
     if (mode == 2) return 256;
-    if (max_nv > 2560) return mode == 1 ? 512 : 768;
-    if (max_nv > 1024 || (few && max_nv > 64)) return 512;
+    if (mode == 1) return 512;
+    if (max_nv > (few ? 512 : 1536)) return 768;
+    if (few && max_nv > 64) return 512;
     return max_nv <= 256 ? 128 : 256;
 }
 
@@ -1486,6 +1490,7 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
         c.scratch_stride = (c.scratch_stride + 255) & ~(size_t)255;
         c.members = (int)mem.size();
         int want = block_override > 0 ? block_override : default_block(c.max_nv, c.mode, N <= few_envs(b));
+        if (accum != FFSRL_ACC_FIXED && block_override <= 0 && c.max_nv <= 2560) want = std::min(want, 512);  // 768 are not built
         if (c.split > 1) {
             int items = 0;
             for (int e : mem)
