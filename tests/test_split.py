@@ -71,3 +71,40 @@ def test_autotuned_split_plan(gpu, tmp_path, monkeypatch):
         torch.cuda.synchronize()
         out.append(m.vertex.cpu().numpy())
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("arithmetic", ["reference", "fast"])
+def test_classes_of_a_step_in_turn(gpu, arithmetic):
+    # each class's kernel waits for the one ahead to have begun: a class left out breaks no
+    # chain, a captured step keeps it, and the envs' bits do not depend on it
+    sizes = (12000, 6000, 2500, 300)
+    meshes = [mg.ellipsoid_for_tets(t, seed=4) for t in sizes]
+
+    def fresh():
+        m, _ = sc.liver_model("cuda:0", len(sizes), meshes=meshes)
+        return m, SimIntegratorDO("cuda:0", arithmetic=arithmetic).plan(m)
+
+    m, plan = fresh()
+    rest = m.vertex.clone()
+    assert plan.info()["num_classes"] > 2
+    for _ in range(3):
+        plan.step(1)
+    torch.cuda.synchronize()
+    want = m.vertex.clone()
+    m, plan = fresh()
+    for _ in range(3):
+        plan.step_envs([0, 2])
+    torch.cuda.synchronize()
+    for e in range(len(sizes)):
+        s = m.envSlice(e)
+        assert torch.equal(m.vertex[s], (want if e in (0, 2) else rest)[s])
+    m, plan = fresh()
+    plan.step(1)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.step(1)
+    graph.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(m.vertex, want)
