@@ -1,7 +1,8 @@
-// plain.cu -- reference-shaped step: one kernel launch per reference kernel, in the
-// launch order of SimIntegratorDO.stepModel (FF_SRL/FF_SRL/integrator.py:1640-1741),
-// per-vertex corrections accumulated with float atomics as the reference does.  This is
-// the drop-in that the batched form (batched.cu) is measured against.
+// plain.cu -- reference-shaped step: the kernels of SimIntegratorDO.stepModel
+// (FF_SRL/FF_SRL/integrator.py:1640-1741) over all envs, in its launch order, per-vertex
+// corrections accumulated with float atomics as the reference does; kernels of it that do not
+// read what the one before writes to other vertices share a launch.  This is the drop-in that
+// the batched form (batched.cu) is measured against.
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <mutex>
@@ -14,14 +15,15 @@ namespace {
 
 constexpr int kBlock = 256;
 
-// The step's some 70 launches a substep are short, so each is allowed to start while the one
+// The step's some 40 launches a substep are short, so each is allowed to start while the one
 // before it is still running (programmatic dependent launch).  Every kernel of the step first
 // lets the next one start, loads what no kernel of the step writes (indices, rest values,
 // masses, flags, the instrument), and then waits -- every thread, so that a kernel cannot
 // complete before the one ahead of it has -- until the writes of the one before are seen.
 // The step's first launch starts after all earlier work, as usual.  A step of 8 x 10
-// iterations took 3,234 us on one mixed env, 4,382 on 16 and 19.8 ms on 256; it takes 1,737,
-// 3,296 and 17.9 ms.  What is left is each kernel's chain of loads and atomics.
+// iterations took 3,234 us on one mixed env, 4,382 on 16 and 19.8 ms on 256; with the early
+// starts 1,737, 3,296 and 17.9 ms, with the shared launches (7 an iteration became 4) 1,186,
+// 1,907 and 12.1 ms.  What is left is each kernel's chain of loads and atomics.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Loads of what the step's kernels write: kept behind the wait (a load through a const
@@ -68,38 +70,6 @@ __global__ void k_gravity(const float* x, float* xp, const float* vel,
     st3(xp, i, p + v * dt);
 }
 
-// volumeConstraints (integrator.py:444-504)
-__global__ void k_volume(const float* xp, float* dp, int* cnt, const int* __restrict__ tet,
-                         const float* __restrict__ rest, const float* __restrict__ inv_mass,
-                         const float* __restrict__ active_tet, float ks, int n) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_start();
-    float active = 0.0f, rv = 0.0f, mA = 0.0f, mB = 0.0f, mC = 0.0f, mD = 0.0f;
-    int4 id = make_int4(0, 0, 0, 0);
-    if (t < n) {
-        active = active_tet[t];
-        id = reinterpret_cast<const int4*>(tet)[t];
-        rv = rest[t];
-        mA = inv_mass[id.x]; mB = inv_mass[id.y]; mC = inv_mass[id.z]; mD = inv_mass[id.w];
-    }
-    wait_for_previous();
-    if (t >= n || !(active == 1.0f)) return;
-    v3 pa = ldw3(xp, id.x), pb = ldw3(xp, id.y), pc = ldw3(xp, id.z), pd = ldw3(xp, id.w);
-    v3 p1 = pb - pa, p2 = pc - pa, p3 = pd - pa;
-    v3 q2 = cross(p3, p1), q1 = cross(p2, p3), q3 = cross(p1, p2);
-    v3 q0 = -q1 - q2 - q3;
-    float vol = fabsf(dot(cross(p1, p2), p3)) / 6.0f;
-    float w = mA * dot(q0, q0) + mB * dot(q1, q1) + mC * dot(q2, q2) + mD * dot(q3, q3);
-    if (fabsf(w) < FFSRL_FLOAT_EPS) return;
-    float C = rv - vol;
-    float dl = -ks * active * C / w;
-    atomic_add3_pair(dp, id.x, q0 * dl * mA);
-    atomic_add3_pair(dp, id.y, q1 * dl * mB);
-    atomic_add3_pair(dp, id.z, q2 * dl * mC);
-    atomic_add3_pair(dp, id.w, q3 * dl * mD);
-    atomicAdd(cnt + id.x, 1); atomicAdd(cnt + id.y, 1); atomicAdd(cnt + id.z, 1); atomicAdd(cnt + id.w, 1);
-}
-
 // volumeConstraintsXPBD (integrator.py:507-576), signed rest volume
 __global__ void k_volume_xpbd(const float* xp, float* dp, int* cnt, float* lam,
                               const int* __restrict__ tet, const float* __restrict__ rest,
@@ -135,93 +105,133 @@ __global__ void k_volume_xpbd(const float* xp, float* dp, int* cnt, float* lam,
     atomicAdd(cnt + id.x, 1); atomicAdd(cnt + id.y, 1); atomicAdd(cnt + id.z, 1); atomicAdd(cnt + id.w, 1);
 }
 
-// neoHookeanConstraints (integrator.py:578-698): stable Neo-Hookean hydrostatic +
-// deviatoric pair with F = [p1 p2 p3] Dm^-1; lambda starts at 0 every projection
-// because the reference never stores it.
-__global__ void k_neohookean(const float* xp, float* dp, int* cnt, const int* __restrict__ tet,
-                             const float* __restrict__ rest, const float* __restrict__ inv_mass,
-                             const float* __restrict__ dm_inv, float vol_c, float dev_c, float dt, int n) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_start();
-    const int tt = t < n ? t : 0;  // (n > 0: a thread past the end loads the first tet's)
-    int4 id = reinterpret_cast<const int4*>(tet)[tt];
-    float rv = rest[tt];
-    float mA = inv_mass[id.x], mB = inv_mass[id.y], mC = inv_mass[id.z], mD = inv_mass[id.w];
-    const float* D = dm_inv + 9ll * tt;
-    float d00 = D[0], d01 = D[1], d02 = D[2], d10 = D[3], d11 = D[4], d12 = D[5], d20 = D[6], d21 = D[7], d22 = D[8];
-    wait_for_previous();
-    if (t >= n) return;
-    v3 pa = ldw3(xp, id.x), pb = ldw3(xp, id.y), pc = ldw3(xp, id.z), pd = ldw3(xp, id.w);
-    v3 p1 = pb - pa, p2 = pc - pa, p3 = pd - pa;
-    v3 f0 = p1 * d00 + p2 * d10 + p3 * d20;
-    v3 f1 = p1 * d01 + p2 * d11 + p3 * d21;
-    v3 f2 = p1 * d02 + p2 * d12 + p3 * d22;
-    v3 c0 = cross(f1, f2), c1 = cross(f2, f0), c2 = cross(f0, f1);
-    v3 g1 = c0 * d00 + c1 * d01 + c2 * d02;
-    v3 g2 = c0 * d10 + c1 * d11 + c2 * d12;
-    v3 g3 = c0 * d20 + c1 * d21 + c2 * d22;
-    v3 g0 = -g1 - g2 - g3;
-    float detF = dot(f0, c0);
-    float invVol = 1.0f / vol_c, invDev = 1.0f / dev_c;
-    float C = detF - 1.0f - invDev / invVol;
-    float w = 0.0f, l;
-    l = length(g0); w += l * l * mA;
-    l = length(g1); w += l * l * mB;
-    l = length(g2); w += l * l * mC;
-    l = length(g3); w += l * l * mD;
-    if (w < FFSRL_FLOAT_EPS) return;
-    float alpha = vol_c / dt / dt / rv;
-    float dl = -C / (w + alpha);
-    v3 dA = g0 * dl * mA, dB = g1 * dl * mB, dC = g2 * dl * mC, dD = g3 * dl * mD;
-    float l0 = length(f0), l1 = length(f1), l2 = length(f2);
-    float rs = sqrtf(l0 * l0 + l1 * l1 + l2 * l2);
-    float rsi = 1.0f / rs;
-    C = rs;
-    g1 = (f0 * d00 + f1 * d01 + f2 * d02) * rsi;
-    g2 = (f0 * d10 + f1 * d11 + f2 * d12) * rsi;
-    g3 = (f0 * d20 + f1 * d21 + f2 * d22) * rsi;
-    g0 = -g1 - g2 - g3;
-    w = 0.0f;
-    l = length(g0); w += l * l * mA;
-    l = length(g1); w += l * l * mB;
-    l = length(g2); w += l * l * mC;
-    l = length(g3); w += l * l * mD;
-    if (w < FFSRL_FLOAT_EPS) return;
-    alpha = dev_c / dt / dt / rv;
-    dl = -C / (w + alpha);
-    dA = dA + g0 * dl * mA; dB = dB + g1 * dl * mB; dC = dC + g2 * dl * mC; dD = dD + g3 * dl * mD;
-    atomic_add3_pair(dp, id.x, dA); atomic_add3_pair(dp, id.y, dB); atomic_add3_pair(dp, id.z, dC); atomic_add3_pair(dp, id.w, dD);
-    atomicAdd(cnt + id.x, 1); atomicAdd(cnt + id.y, 1); atomicAdd(cnt + id.z, 1); atomicAdd(cnt + id.w, 1);
-}
-
-// distanceConstraints (integrator.py:65-109)
-__global__ void k_distance(const float* xp, float* dp, int* cnt, const int* __restrict__ edge,
-                           const float* __restrict__ rest, const float* __restrict__ inv_mass,
-                           const float* __restrict__ active_edge, float ks, int n) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_start();
-    float active = 0.0f, L0 = 0.0f, mA = 0.0f, mB = 0.0f;
-    int2 id = make_int2(0, 0);
-    if (e < n) {
-        active = active_edge[e];
-        id = reinterpret_cast<const int2*>(edge)[e];
-        L0 = rest[e];
-        mA = inv_mass[id.x]; mB = inv_mass[id.y];
+// The volume, Neo-Hookean and distance constraints of one projection, in one launch: its
+// first blocks take a tet a thread, the others an edge a thread.
+// volumeConstraints (integrator.py:444-504); neoHookeanConstraints (:578-698): hydrostatic +
+// deviatoric pair with F = [p1 p2 p3] Dm^-1; lambda starts at 0 every projection because the
+// reference never stores it; distanceConstraints (:65-109).
+// All three read the same positions and add to the same sums, in any order.  A launch of
+// their own cost each some 5 us however small it was, and a tet's two constraints read the
+// same vertices and added to the same sums twice (256 envs of 500-20,000 tets: 16.2 ms a step
+// with a launch each, 12.1 so).
+struct Tets {
+    const int* tet;
+    const float *rest, *active, *dm_inv;
+    float ks, vol_c, dev_c, dt;
+    int n;
+};
+struct Edges {
+    const int* edge;
+    const float *rest, *active;
+    float ks;
+    int n;
+};
+__device__ __forceinline__ void tet_constraints(const float* xp, float* dp, int* cnt, const float* __restrict__ inv_mass,
+                                                const Tets& a, bool volume, bool neo, int t) {
+    const int tt = t < a.n ? t : 0;  // (n > 0: a thread past the end loads the first tet's)
+    const int4 id = __ldg(reinterpret_cast<const int4*>(a.tet) + tt);
+    const float rv = __ldg(a.rest + tt), active = volume ? __ldg(a.active + tt) : 0.0f;
+    const float mA = __ldg(inv_mass + id.x), mB = __ldg(inv_mass + id.y), mC = __ldg(inv_mass + id.z), mD = __ldg(inv_mass + id.w);
+    float d00 = 0.0f, d01 = 0.0f, d02 = 0.0f, d10 = 0.0f, d11 = 0.0f, d12 = 0.0f, d20 = 0.0f, d21 = 0.0f, d22 = 0.0f;
+    if (neo) {
+        const float* D = a.dm_inv + 9ll * tt;
+        d00 = __ldg(D); d01 = __ldg(D + 1); d02 = __ldg(D + 2); d10 = __ldg(D + 3); d11 = __ldg(D + 4); d12 = __ldg(D + 5);
+        d20 = __ldg(D + 6); d21 = __ldg(D + 7); d22 = __ldg(D + 8);
     }
     wait_for_previous();
-    if (e >= n || active == 0.0f) return;
+    if (t >= a.n || (!neo && !(active == 1.0f))) return;
+    const v3 pa = ldw3(xp, id.x), pb = ldw3(xp, id.y), pc = ldw3(xp, id.z), pd = ldw3(xp, id.w);
+    const v3 p1 = pb - pa, p2 = pc - pa, p3 = pd - pa;
+    v3 dA = mk(0.0f, 0.0f, 0.0f), dB = dA, dC = dA, dD = dA;
+    int k = 0;
+    if (active == 1.0f) {
+        const v3 q2 = cross(p3, p1), q1 = cross(p2, p3), q3 = cross(p1, p2);
+        const v3 q0 = -q1 - q2 - q3;
+        const float vol = fabsf(dot(q3, p3)) / 6.0f;
+        const float w = mA * dot(q0, q0) + mB * dot(q1, q1) + mC * dot(q2, q2) + mD * dot(q3, q3);
+        if (!(fabsf(w) < FFSRL_FLOAT_EPS)) {
+            const float C = rv - vol;
+            const float dl = -a.ks * active * C / w;
+            dA = q0 * dl * mA; dB = q1 * dl * mB; dC = q2 * dl * mC; dD = q3 * dl * mD;
+            ++k;
+        }
+    }
+    if (neo) {
+        const v3 f0 = p1 * d00 + p2 * d10 + p3 * d20;
+        const v3 f1 = p1 * d01 + p2 * d11 + p3 * d21;
+        const v3 f2 = p1 * d02 + p2 * d12 + p3 * d22;
+        const v3 c0 = cross(f1, f2), c1 = cross(f2, f0), c2 = cross(f0, f1);
+        v3 g1 = c0 * d00 + c1 * d01 + c2 * d02;
+        v3 g2 = c0 * d10 + c1 * d11 + c2 * d12;
+        v3 g3 = c0 * d20 + c1 * d21 + c2 * d22;
+        v3 g0 = -g1 - g2 - g3;
+        const float detF = dot(f0, c0);
+        const float invVol = 1.0f / a.vol_c, invDev = 1.0f / a.dev_c;
+        float C = detF - 1.0f - invDev / invVol;
+        float w = 0.0f, l;
+        l = length(g0); w += l * l * mA;
+        l = length(g1); w += l * l * mB;
+        l = length(g2); w += l * l * mC;
+        l = length(g3); w += l * l * mD;
+        if (!(w < FFSRL_FLOAT_EPS)) {
+            float alpha = a.vol_c / a.dt / a.dt / rv;
+            float dl = -C / (w + alpha);
+            v3 nA = g0 * dl * mA, nB = g1 * dl * mB, nC = g2 * dl * mC, nD = g3 * dl * mD;
+            const float l0 = length(f0), l1 = length(f1), l2 = length(f2);
+            const float rs = sqrtf(l0 * l0 + l1 * l1 + l2 * l2);
+            const float rsi = 1.0f / rs;
+            C = rs;
+            g1 = (f0 * d00 + f1 * d01 + f2 * d02) * rsi;
+            g2 = (f0 * d10 + f1 * d11 + f2 * d12) * rsi;
+            g3 = (f0 * d20 + f1 * d21 + f2 * d22) * rsi;
+            g0 = -g1 - g2 - g3;
+            w = 0.0f;
+            l = length(g0); w += l * l * mA;
+            l = length(g1); w += l * l * mB;
+            l = length(g2); w += l * l * mC;
+            l = length(g3); w += l * l * mD;
+            if (!(w < FFSRL_FLOAT_EPS)) {
+                alpha = a.dev_c / a.dt / a.dt / rv;
+                dl = -C / (w + alpha);
+                nA = nA + g0 * dl * mA; nB = nB + g1 * dl * mB; nC = nC + g2 * dl * mC; nD = nD + g3 * dl * mD;
+                dA = dA + nA; dB = dB + nB; dC = dC + nC; dD = dD + nD;
+                ++k;
+            }
+        }
+    }
+    if (!k) return;
+    atomic_add3_pair(dp, id.x, dA); atomic_add3_pair(dp, id.y, dB); atomic_add3_pair(dp, id.z, dC); atomic_add3_pair(dp, id.w, dD);
+    atomicAdd(cnt + id.x, k); atomicAdd(cnt + id.y, k); atomicAdd(cnt + id.z, k); atomicAdd(cnt + id.w, k);
+}
+__device__ __forceinline__ void edge_constraint(const float* xp, float* dp, int* cnt, const float* __restrict__ inv_mass,
+                                                const Edges& a, int e) {
+    const int ee = e < a.n ? e : 0;
+    const float active = __ldg(a.active + ee), L0 = __ldg(a.rest + ee);
+    const int2 id = __ldg(reinterpret_cast<const int2*>(a.edge) + ee);
+    const float mA = __ldg(inv_mass + id.x), mB = __ldg(inv_mass + id.y);
+    wait_for_previous();
+    if (e >= a.n || active == 0.0f) return;
     if (L0 < FFSRL_FLOAT_EPS) return;
-    v3 pa = ldw3(xp, id.x), pb = ldw3(xp, id.y);
-    v3 dir = pb - pa;
-    float len = length(dir);
+    const v3 pa = ldw3(xp, id.x), pb = ldw3(xp, id.y);
+    const v3 dir = pb - pa;
+    const float len = length(dir);
     if (len < FFSRL_FLOAT_EPS) return;
-    float w = mA + mB;
+    const float w = mA + mB;
     if (w < FFSRL_FLOAT_EPS) return;
-    float C = len - L0;
-    v3 d = -C * (dir / len) * ks * active / w;
+    const float C = len - L0;
+    const v3 d = -C * (dir / len) * a.ks * active / w;
     atomic_add3_pair(dp, id.x, -(d * mA));
     atomic_add3_pair(dp, id.y, d * mB);
     atomicAdd(cnt + id.x, 1); atomicAdd(cnt + id.y, 1);
+}
+__global__ void k_constraints(const float* xp, float* dp, int* cnt, const float* __restrict__ inv_mass, Tets tets, Edges edges,
+                              unsigned tet_blocks, unsigned fl) {
+    let_next_start();
+    if (blockIdx.x < tet_blocks)
+        tet_constraints(xp, dp, cnt, inv_mass, tets, (fl & FFSRL_VOLUME) != 0, (fl & FFSRL_NEOHOOKEAN) != 0,
+                        blockIdx.x * blockDim.x + threadIdx.x);
+    else
+        edge_constraint(xp, dp, cnt, inv_mass, edges, (blockIdx.x - tet_blocks) * blockDim.x + threadIdx.x);
 }
 
 // distanceConstraintsXPBD (integrator.py:191-240)
@@ -258,38 +268,37 @@ __global__ void k_distance_xpbd(const float* xp, float* dp, int* cnt, float* lam
     atomicAdd(cnt + id.x, 1); atomicAdd(cnt + id.y, 1);
 }
 
-// applyConstraints (integrator.py:946-960)
-__global__ void k_apply(float* xp, float* dp, int* cnt, int n) {
+// applyConstraints (integrator.py:946-960), then dragConstraintsDO (:412-442): pull toward
+// laparoscopeTip[env*4 + 2] (drag null: none).  Both touch a thread's own vertex alone.
+__global__ void k_apply(float* xp, float* dp, int* cnt, const float* __restrict__ drag, const int* __restrict__ v2e,
+                        const float* __restrict__ tip, float ks, int n) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     let_next_start();
-    wait_for_previous();
-    if (i >= n) return;
-    const v3 d = ldw3(dp, i), x = ldw3(xp, i);
-    int c = __float_as_int(ldw(reinterpret_cast<const float*>(cnt + i)));
-    if (c > 0) {
-        float N = float(c);
-        st3(xp, i, x + mk(d.x / N, d.y / N, d.z / N));
-    }
-    st3(dp, i, mk(0.0f, 0.0f, 0.0f));
-    cnt[i] = 0;
-}
-
-// dragConstraintsDO (integrator.py:412-442): pull toward laparoscopeTip[env*4 + 2]
-__global__ void k_drag(float* xp, const float* __restrict__ drag, const int* __restrict__ v2e,
-                       const float* __restrict__ tip, float ks, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_start();
-    float dr = i < n ? drag[i] : 0.0f;
+    const float dr = i < n && drag ? drag[i] : 0.0f;
     v3 t = mk(0.0f, 0.0f, 0.0f);
     if (dr != 0.0f) t = ld3(tip, 4ll * v2e[i] + 2);
     wait_for_previous();
-    if (i >= n || dr == 0.0f) return;
-    v3 pos = ldw3(xp, i);
-    v3 dir = pos - t;
-    float len = length(dir);
-    if (len < FFSRL_FLOAT_EPS) return;
-    v3 d = len * normalize(dir) * dr * ks / 2.0f;
-    st3(xp, i, pos - d);
+    if (i >= n) return;
+    const v3 d = ldw3(dp, i);
+    v3 x = ldw3(xp, i);
+    int c = __float_as_int(ldw(reinterpret_cast<const float*>(cnt + i)));
+    bool moved = false;
+    if (c > 0) {
+        float N = float(c);
+        x = x + mk(d.x / N, d.y / N, d.z / N);
+        moved = true;
+    }
+    if (dr != 0.0f) {
+        const v3 dir = x - t;
+        const float len = length(dir);
+        if (!(len < FFSRL_FLOAT_EPS)) {
+            x = x - len * normalize(dir) * dr * ks / 2.0f;
+            moved = true;
+        }
+    }
+    if (moved) st3(xp, i, x);
+    st3(dp, i, mk(0.0f, 0.0f, 0.0f));
+    cnt[i] = 0;
 }
 
 // triToPointDistanceConstraintsDO (integrator.py:300-353)
@@ -390,22 +399,17 @@ __global__ void k_collide_apply(float* xp, float* cdp, int n) {
     st3(cdp, i, mk(0.0f, 0.0f, 0.0f));
 }
 
-// bounds (integrator.py:12-21)
-__global__ void k_bounds(float* xp, float ground, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    let_next_start();
-    wait_for_previous();
-    if (i >= n) return;
-    if (ldw(xp + 3 * i + 1) < ground) xp[3 * i + 1] = ground;
-}
-
-// PBDStep (integrator.py:23-38)
-__global__ void k_pbd(float* x, const float* xp, float* vel, float dt, int n) {
+// bounds (integrator.py:12-21), then PBDStep (:23-38)
+__global__ void k_finish(float* x, float* xp, float* vel, float ground, float dt, int n) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     let_next_start();
     wait_for_previous();
     if (i >= n) return;
     v3 p = ldw3(x, i), q = ldw3(xp, i);
+    if (q.y < ground) {
+        q.y = ground;
+        xp[3 * i + 1] = ground;
+    }
     v3 v = (q - p) * (1.0f / dt);
     st3(x, i, q);
     st3(vel, i, v);
@@ -591,6 +595,10 @@ extern "C" int32_t ffsrl_step_model(const ffsrl_model* m, const ffsrl_params* p,
     const float avol = (float)((double)p->volume_compliance_xpbd / ((double)p->dt * (double)p->dt));
     const unsigned gv = grid_for(V, kBlock), gt = grid_for(T, kBlock), ge = grid_for(E, kBlock);
     const unsigned gf = grid_for(F, kBlock), gc = grid_for(C, kBlock);
+    const unsigned nt = (fl & (FFSRL_VOLUME | FFSRL_NEOHOOKEAN)) && T > 0 ? gt : 0, ne = (fl & FFSRL_DISTANCE) && E > 0 ? ge : 0;
+    const Tets tets{m->tetrahedron, m->tetrahedron_rest_volume, m->active_tetrahedron, m->tetrahedron_dm_inv,
+                    p->ks_volume, p->volume_compliance, p->deviatoric_compliance, p->dt, T};
+    const Edges edges{m->edge, m->edge_rest_length, m->active_edge, p->ks_distance, E};
     cudaError_t err = cudaSuccess;
     bool first = true;
     auto go = [&](auto k, unsigned grid, auto... args) {
@@ -603,30 +611,18 @@ extern "C" int32_t ffsrl_step_model(const ffsrl_model* m, const ffsrl_params* p,
         if ((fl & FFSRL_DISTANCE_XPBD) && E > 0) go(k_zero, ge, m->edge_lambda, E);
         if ((fl & FFSRL_VOLUME_XPBD) && T > 0) go(k_zero, gt, m->tetrahedron_lambda, T);
         for (int it = 0; it < p->iterations; ++it) {
-            if ((fl & FFSRL_VOLUME) && T > 0)
-                go(k_volume, gt, m->predicted_vertex, m->dp, m->constraints_number, m->tetrahedron,
-                   m->tetrahedron_rest_volume, m->inverse_mass, m->active_tetrahedron,
-                   p->ks_volume, T);
+            if (nt + ne > 0)
+                go(k_constraints, nt + ne, m->predicted_vertex, m->dp, m->constraints_number, m->inverse_mass, tets, edges, nt, fl);
             if ((fl & FFSRL_VOLUME_XPBD) && T > 0)
                 go(k_volume_xpbd, gt, m->predicted_vertex, m->dp, m->constraints_number,
                    m->tetrahedron_lambda, m->tetrahedron, m->xpbd_rest_volume,
                    m->inverse_mass, m->active_tetrahedron, avol, T);
-            if ((fl & FFSRL_NEOHOOKEAN) && T > 0)
-                go(k_neohookean, gt, m->predicted_vertex, m->dp, m->constraints_number, m->tetrahedron,
-                   m->tetrahedron_rest_volume, m->inverse_mass, m->tetrahedron_dm_inv,
-                   p->volume_compliance, p->deviatoric_compliance, p->dt, T);
-            if ((fl & FFSRL_DISTANCE) && E > 0)
-                go(k_distance, ge, m->predicted_vertex, m->dp, m->constraints_number, m->edge,
-                   m->edge_rest_length, m->inverse_mass, m->active_edge, p->ks_distance,
-                   E);
             if ((fl & FFSRL_DISTANCE_XPBD) && E > 0)
                 go(k_distance_xpbd, ge, m->predicted_vertex, m->dp, m->constraints_number,
                    m->edge_lambda, m->edge, m->edge_rest_length, m->inverse_mass,
                    m->active_edge, adist, E);
-            go(k_apply, gv, m->predicted_vertex, m->dp, m->constraints_number, V);
-            if (fl & FFSRL_DRAG)
-                go(k_drag, gv, m->predicted_vertex, m->active_drag_constraint, m->vertex_to_env,
-                   m->laparoscope_tip, p->ks_drag, V);
+            go(k_apply, gv, m->predicted_vertex, m->dp, m->constraints_number, (fl & FFSRL_DRAG) ? m->active_drag_constraint : nullptr,
+               m->vertex_to_env, m->laparoscope_tip, p->ks_drag, V);
             if ((fl & FFSRL_CONNECTORS) && C > 0)
                 go(k_connector, gc, m->predicted_vertex, m->dp, m->constraints_number,
                    m->connector_triangle_id, m->connector_tri_bar,
@@ -640,8 +636,7 @@ extern "C" int32_t ffsrl_step_model(const ffsrl_model* m, const ffsrl_params* p,
                 go(k_collide_apply, gv, m->predicted_vertex, m->collision_dp, V);
             }
         }
-        go(k_bounds, gv, m->predicted_vertex, p->ground_level, V);
-        go(k_pbd, gv, m->vertex, m->predicted_vertex, m->velocity, p->dt, V);
+        go(k_finish, gv, m->vertex, m->predicted_vertex, m->velocity, p->ground_level, p->dt, V);
     }
     if (err != cudaSuccess) cudaGetLastError();  // (the launch has recorded it, too)
     if (err != cudaSuccess) return cuda_fail(err, "ffsrl_step_model");
