@@ -810,8 +810,8 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
                 // Dm^-1 as stored (row-major), read by the reference-form kernel as the
                 // reference reads it
                 const float* f = hm->tetrahedron_dm_inv + 9ll * t;
-                nhd[3 * t] = make_float4(f[0], f[1], f[2], f[3]);
-                nhd[3 * t + 1] = make_float4(f[4], f[5], f[6], f[7]);
+                nhd[3 * t] = make_float4(f[0], f[1], f[3], f[4]);
+                nhd[3 * t + 1] = make_float4(f[6], f[7], f[2], f[5]);
                 const float v0 = tet_va[t].x;
                 nhd[3 * t + 2] = make_float4(f[8], p->volume_compliance / p->dt / p->dt / v0,
                                              p->deviatoric_compliance / p->dt / p->dt / v0,

@@ -55,7 +55,7 @@ __device__ Out plain(unsigned fl, const TetRec& rc, const float4* x, bool fold, 
         }
     }
     if (fl & FFSRL_NEOHOOKEAN) {
-        const float D[3][3] = {{rc.n0.x, rc.n0.y, rc.n0.z}, {rc.n0.w, rc.n1.x, rc.n1.y}, {rc.n1.z, rc.n1.w, rc.n2.x}};
+        const float D[3][3] = {{rc.n0.x, rc.n0.y, rc.n1.z}, {rc.n0.z, rc.n0.w, rc.n1.w}, {rc.n1.x, rc.n1.y, rc.n2.x}};
         V f[3], c[3], g[4], n[4];
         for (int j = 0; j < 3; ++j) f[j] = p1 * D[0][j] + p2 * D[1][j] + p3 * D[2][j];
         c[0] = cross(f[1], f[2]); c[1] = cross(f[2], f[0]); c[2] = cross(f[0], f[1]);
