@@ -11,7 +11,7 @@ and a 128x128 (2x2 supersampled) depth + colour ray-cast per environment.
   e2e    -- the same through the public API with host buffers: each step copies the
             actions (N x 4 float32 from pinned memory) to the device and reads back the
             per-env result (effector position + contact count, N x 4 float32)
-  plain  -- the reference-shaped drop-in (one launch per reference kernel) on the same GPU
+  plain  -- the reference-shaped drop-in (the reference's kernels over all envs) on the same GPU
 
 Every env has a mesh of its own by default (config 2 draws a tet count per env);
 ``--pool K`` draws the 4096 envs from K shared meshes instead.  ``--arithmetic`` picks the
@@ -470,8 +470,8 @@ def main():
                    "sample": f"32 envs of the same pool, 1 full env-step (8x10 solve, refit, {RES}x{RES} ray-cast), "
                              "oracle restatement, OpenMP over envs"}
         # per step: instrument kinematics, one launch per size class, remap, instrument visual points,
-        # fused refit, normal gather, rays; per episode reset: instrument visual points, remap and grasp
-        launches = K * (n_cls + 6) + 3 * resets_timed
+        # fused refit (leaves, then the climb), normal gather, rays; per episode reset: instrument visual points, remap and grasp
+        launches = K * (n_cls + 7) + 3 * resets_timed
         line = {"metric": METRIC, "value": value, "unit": "env-steps/s", "n_gpus": world, "steps": K,
                 "warmup": W, "ms_per_step": total_ms / K, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded meshes and random-walk actions)",

@@ -7,15 +7,16 @@ onto the visual points (``transformSimMeshData``), as the reference does.
 Two GPU forms with the same semantics:
 
 * ``batched=True`` (default): the env-resident batched kernel -- one persistent launch per
-  mesh-size class, every substep and iteration of an environment on one SM, shared-memory
+  mesh-size class, every substep and iteration of an environment on one SM (on a
+  cluster of SMs where the environments are few), shared-memory
   positions and deterministic fixed-point correction sums.  ``arithmetic="reference"``
   (default) evaluates every constraint with the reference kernel's expressions (IEEE
   division and square root, no fused multiply-add); ``"fast"`` uses hardware
   reciprocals and a reformulated Neo-Hookean constraint.  ``accumulation`` selects
   ``"fixed"`` (default), ``"kahan"`` (compensated float32) or ``"atomic"`` (float32
   atomics, as the reference);
-* ``batched=False``: the reference-shaped form -- one kernel launch per reference kernel
-  in the reference's launch order, float atomics.
+* ``batched=False``: the reference-shaped form -- the reference's kernels over all
+  environments, in its order, float atomics.
 """
 
 from __future__ import annotations

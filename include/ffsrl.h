@@ -204,7 +204,7 @@ int32_t ffsrl_device_info(int32_t* sm_count, int32_t* max_smem_per_block, int32_
 
 /* One SimIntegratorDO.stepModel (integrator.py:1640-1741): substeps x (gravity,
    iterations x (constraints, applyConstraints, drag, connectors, collide), bounds,
-   PBDStep), one kernel launch per reference kernel, float atomics as the reference. */
+   PBDStep): the reference's kernels over all envs, float atomics as the reference. */
 int32_t ffsrl_step_model(const ffsrl_model* model, const ffsrl_params* params, void* stream);
 
 /* No counterpart in the reference.  ffsrl_step_model for callers that cannot allocate
@@ -382,14 +382,17 @@ int32_t ffsrl_batch_step_envs_lane(ffsrl_batch* b, int32_t lane, const int32_t* 
 int32_t ffsrl_batch_info(const ffsrl_batch* b, int64_t* device_bytes, int32_t* num_classes, int32_t* block_threads);
 /* Size classes (environments grouped by vertex count, one launch each): the class's
    largest vertex count, storage mode (0 shared, 1 shared positions + global sums,
-   2 global), block size and environment count; its env ids; its block size. */
+   2 global), block size and environment count; its env ids; its block size.  In plans of
+   few envs a class's envs may each be divided among a cluster of blocks: the class keeps the
+   sums in shared memory then, and vertex count and mode are those of an undivided env. */
 int32_t ffsrl_batch_class_info(const ffsrl_batch* b, int32_t cls, int32_t* max_nv, int32_t* mode, int32_t* block,
                                int32_t* num_envs);
 int32_t ffsrl_batch_class_envs(const ffsrl_batch* b, int32_t cls, int32_t* env_ids);
 int32_t ffsrl_batch_set_class_block(ffsrl_batch* b, int32_t cls, int32_t block);
 /* Autotuner hook, how class cls's kernel fetches each thread's next tet record one loop
    trip ahead: 0 not at all, 1 into L1 (prefetch.global.L1), 2 into registers (block sizes
-   512 and 640, float32).  Results are unchanged.  A kind the class's block size has no
+   512 and 640, float32).  Results are unchanged.  A class whose envs are divided among
+   blocks takes any kind, and fetches in one way.  A kind the class's block size has no
    kernel for is refused and leaves the class as it was. */
 int32_t ffsrl_batch_set_class_prefetch(ffsrl_batch* b, int32_t cls, int32_t kind);
 /* Copies the float64 plan's state (x, v, predicted, each [3V]) to host memory. */
