@@ -14,6 +14,7 @@ namespace ffsrl {
 namespace {
 
 constexpr int kBlock = 256;
+constexpr int kFourLanes = 100000;  // the most triangles k_collide takes four lanes each for
 
 // The step's some 40 launches a substep are short, so each is allowed to start while the one
 // before it is still running (programmatic dependent launch).  Every kernel of the step first
@@ -23,7 +24,8 @@ constexpr int kBlock = 256;
 // The step's first launch starts after all earlier work, as usual.  A step of 8 x 10
 // iterations took 3,234 us on one mixed env, 4,382 on 16 and 19.8 ms on 256; with the early
 // starts 1,737, 3,296 and 17.9 ms, with the shared launches (7 an iteration became 4) 1,186,
-// 1,907 and 12.1 ms.  What is left is each kernel's chain of loads and atomics.
+// 1,907 and 12.1 ms, with four lanes a triangle in the contact 868, 1,600 and 12.1.  What is
+// left is each kernel's chain of loads and atomics.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Loads of what the step's kernels write: kept behind the wait (a load through a const
@@ -333,12 +335,21 @@ __global__ void k_connector(const float* xp, float* dp, int* cnt, const int* __r
 // collideLaparoscopeDO (integrator.py:981-1050).  Responses go to a separate
 // accumulator instead of straight into predictedVertex, so every triangle reads the
 // positions as they were when the launch began; k_collide_apply subtracts them.
+// L lanes a triangle: four, three with a capsule each and the first to add them, or one.  The
+// responses are a chain of square roots and divisions that the few triangles in reach wait
+// for, so small models take four lanes: a step of 8 x 10 iterations on 1, 16 and 64 mixed envs
+// (1,144, 23,168 and 92,672 triangles) takes 868, 1,600 and 3,695 us with four, 1,183, 1,885 and
+// 3,788 with one.  From about 110,000 triangles on the lanes that only scan cost more: 139,008
+// 5.14 ms and 5.07, 370,688 12.9 and 12.1.
+template <int L>
 __global__ void k_collide(const float* xp, float* cdp, const int* __restrict__ tri,
                           const int* __restrict__ t2e, const int* __restrict__ hole,
                           const float* __restrict__ inv_mass, const float* __restrict__ base,
                           const float* __restrict__ tip, const float* __restrict__ radius, int* in_collision,
                           float ks, int n) {
-    int f = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int N = L == 4 ? 1 : 3;  // a lane's capsules
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int f = (int)(g / L), lane = (int)(g % L);
     let_next_start();
     int env = 0, a = 0, b = 0, c = 0;
     bool open = true;
@@ -347,41 +358,61 @@ __global__ void k_collide(const float* xp, float* cdp, const int* __restrict__ t
         open = hole[f] == 1;
         a = tri[3 * f]; b = tri[3 * f + 1]; c = tri[3 * f + 2];
     }
+    auto capsule = [&](int i) { return 4ll * env + (L == 4 ? min(lane, 2) : i); };
     // each capsule's box (its segment lies within a radius of base..tip), and its reach
-    v3 clo[3], chi[3];
-    for (int i = 0; i < 3; ++i) {
-        const long long k = 4ll * env + i;
+    v3 clo[N], chi[N];
+    for (int i = 0; i < N; ++i) {
+        const long long k = capsule(i);
         const v3 p = ld3(base, k), q = ld3(tip, k);
         const float mag = fmaxf(fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(p.z), fabsf(q.x))), fmaxf(fabsf(q.y), fabsf(q.z)));
         const float m = 2.0f * radius[k] + 1e-4f * (1.0f + mag);
         clo[i] = mk(fminf(p.x, q.x) - m, fminf(p.y, q.y) - m, fminf(p.z, q.z) - m);
         chi[i] = mk(fmaxf(p.x, q.x) + m, fmaxf(p.y, q.y) + m, fmaxf(p.z, q.z) + m);
     }
+    Capsule cap = {};
+    if (L == 4) cap = make_capsule(ld3(tip, capsule(0)), ld3(base, capsule(0)), radius[capsule(0)]);
     wait_for_previous();
-    if (open) return;
-    v3 pA = ldw3(xp, a), pB = ldw3(xp, b), pC = ldw3(xp, c);
-    // A response needs a point of the capsule's segment within its radius of a point of the
-    // triangle, so there is none where the boxes are apart (the margin, 1e-4 of the
-    // coordinates, is far above their rounding).  A triangle without one adds nothing.  NaN
-    // coordinates are not apart from anything.
-    const v3 lo = vmin(pA, vmin(pB, pC)), hi = vmax(pA, vmax(pB, pC));
-    const float sum = ((pA.x + pA.y) + (pA.z + pB.x)) + ((pB.y + pB.z) + (pC.x + pC.y)) + pC.z;
+    v3 pA = mk(0.0f, 0.0f, 0.0f), pB = pA, pC = pA;
     unsigned near = 0;
-    for (int i = 0; i < 3; ++i)
-        if (isnan(sum) || !(lo.x > chi[i].x || lo.y > chi[i].y || lo.z > chi[i].z || hi.x < clo[i].x || hi.y < clo[i].y || hi.z < clo[i].z))
-            near |= 1u << i;
-    if (!near) return;
-    v3 centre = (pA + pB + pC) * 0.3333f;
-    v3 nrm = normalize(cross(pB - pA, pC - pA));
+    if (!open) {
+        pA = ldw3(xp, a); pB = ldw3(xp, b); pC = ldw3(xp, c);
+        // A response needs a point of the capsule's segment within its radius of a point of the
+        // triangle, so there is none where the boxes are apart (the margin, 1e-4 of the
+        // coordinates, is far above their rounding).  A triangle without one adds nothing.  NaN
+        // coordinates are not apart from anything.
+        const v3 lo = vmin(pA, vmin(pB, pC)), hi = vmax(pA, vmax(pB, pC));
+        const float sum = ((pA.x + pA.y) + (pA.z + pB.x)) + ((pB.y + pB.z) + (pC.x + pC.y)) + pC.z;
+        for (int i = 0; i < N; ++i)
+            if (isnan(sum) || !(lo.x > chi[i].x || lo.y > chi[i].y || lo.z > chi[i].z || hi.x < clo[i].x || hi.y < clo[i].y || hi.z < clo[i].z))
+                near |= 1u << i;
+        if (L == 4 && lane == 3) near = 0;
+    }
+    if (L == 4 ? !__any_sync(0xffffffffu, near != 0) : !near) return;
+    const v3 centre = (pA + pB + pC) * 0.3333f;
+    const v3 nrm = normalize(cross(pB - pA, pC - pA));
     v3 tA = mk(0.0f, 0.0f, 0.0f), tB = tA, tC = tA;
     float tl = 0.0f;
-    for (int i = 0; i < 3; ++i) {
-        if (!((near >> i) & 1u)) continue;
-        long long k = 4ll * env + i;
+    if (L == 4) {
         v3 rA = mk(0.0f, 0.0f, 0.0f), rB = rA, rC = rA;
-        capsule_response(ld3(tip, k), ld3(base, k), radius[k], nrm, centre, pA, pB, pC, ks, rA, rB, rC);
-        tA = tA + rA; tB = tB + rB; tC = tC + rC;
-        tl = tl + length(rA) + length(rB) + length(rC);
+        if (near) capsule_response(cap, nrm, centre, pA, pB, pC, ks, rA, rB, rC);
+        const float rl = length(rA) + length(rB) + length(rC);
+        for (int j = 0; j < 3; ++j) {
+            auto from = [&](float v) { return __shfl_sync(0xffffffffu, v, j, 4); };
+            tA = tA + mk(from(rA.x), from(rA.y), from(rA.z));
+            tB = tB + mk(from(rB.x), from(rB.y), from(rB.z));
+            tC = tC + mk(from(rC.x), from(rC.y), from(rC.z));
+            tl = tl + from(rl);
+        }
+        if (open || lane != 0) return;
+    } else {
+        for (int i = 0; i < N; ++i) {
+            if (!((near >> i) & 1u)) continue;
+            v3 rA = mk(0.0f, 0.0f, 0.0f), rB = rA, rC = rA;
+            capsule_response(make_capsule(ld3(tip, capsule(i)), ld3(base, capsule(i)), radius[capsule(i)]), nrm, centre, pA, pB, pC, ks,
+                             rA, rB, rC);
+            tA = tA + rA; tB = tB + rB; tC = tC + rC;
+            tl = tl + length(rA) + length(rB) + length(rC);
+        }
     }
     if (tl > 0.0f) atomicAdd(in_collision + env, 1);
     if (!(tl > 0.0f) && !isnan(tl)) return;  // every response is zero
@@ -594,7 +625,7 @@ extern "C" int32_t ffsrl_step_model(const ffsrl_model* m, const ffsrl_params* p,
     const float adist = (float)((double)p->distance_compliance / ((double)p->dt * (double)p->dt));
     const float avol = (float)((double)p->volume_compliance_xpbd / ((double)p->dt * (double)p->dt));
     const unsigned gv = grid_for(V, kBlock), gt = grid_for(T, kBlock), ge = grid_for(E, kBlock);
-    const unsigned gf = grid_for(F, kBlock), gc = grid_for(C, kBlock);
+    const unsigned gc = grid_for(C, kBlock);
     const unsigned nt = (fl & (FFSRL_VOLUME | FFSRL_NEOHOOKEAN)) && T > 0 ? gt : 0, ne = (fl & FFSRL_DISTANCE) && E > 0 ? ge : 0;
     const Tets tets{m->tetrahedron, m->tetrahedron_rest_volume, m->active_tetrahedron, m->tetrahedron_dm_inv,
                     p->ks_volume, p->volume_compliance, p->deviatoric_compliance, p->dt, T};
@@ -630,9 +661,13 @@ extern "C" int32_t ffsrl_step_model(const ffsrl_model* m, const ffsrl_params* p,
                    p->connector_mass_weight_ratio, p->connector_ks,
                    p->connector_rest_length_mul, C);
             if ((fl & FFSRL_COLLIDE) && F > 0) {
-                go(k_collide, gf, m->predicted_vertex, m->collision_dp, m->triangle, m->tri_to_env,
-                   m->hole, m->inverse_mass, m->laparoscope_base, m->laparoscope_tip,
-                   m->laparoscope_radius, m->laparoscope_in_collision, p->ks_contact, F);
+                auto collide = [&](auto k, int lanes) {
+                    go(k, grid_for((long long)lanes * F, kBlock), m->predicted_vertex, m->collision_dp, m->triangle, m->tri_to_env,
+                       m->hole, m->inverse_mass, m->laparoscope_base, m->laparoscope_tip, m->laparoscope_radius,
+                       m->laparoscope_in_collision, p->ks_contact, F);
+                };
+                if (F <= kFourLanes) collide(k_collide<4>, 4);
+                else collide(k_collide<1>, 1);
                 go(k_collide_apply, gv, m->predicted_vertex, m->collision_dp, V);
             }
         }

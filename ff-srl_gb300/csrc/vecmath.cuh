@@ -104,18 +104,27 @@ __device__ __forceinline__ v3 closest_bary(v3 a, v3 b, v3 c, v3 p) {
 
 // checkSdfCapsuleCollision (integrator.py:1302-1355).  Note the reference passes the
 // barycentric triple of the line/plane point (not the point) to closestPointOnEdge.
-__device__ __forceinline__ bool capsule_response(v3 tip, v3 base, float radius, v3 n, v3 centre, v3 pA, v3 pB,
+// The capsule's part of it: the axis and the ends of the segment
+struct Capsule { v3 base, cn, posA, posB; float radius; };
+__device__ __forceinline__ Capsule make_capsule(v3 tip, v3 base, float radius) {
+    Capsule c;
+    c.base = base; c.radius = radius;
+    c.cn = normalize(tip - base);
+    v3 off = c.cn * radius;
+    c.posA = base + off;
+    c.posB = tip - off;
+    return c;
+}
+__device__ __forceinline__ bool capsule_response(const Capsule& k, v3 n, v3 centre, v3 pA, v3 pB,
                                                  v3 pC, float ks, v3& rA, v3& rB, v3& rC) {
-    v3 cn = normalize(tip - base);
-    v3 off = cn * radius;
-    v3 posA = base + off;
-    v3 posB = tip - off;
+    const v3 cn = k.cn, base = k.base;
+    const float radius = k.radius;
     float denom = dot(n, cn);
     if (fabsf(denom) < FFSRL_FLOAT_EPS) return false;
     float t = dot(n, centre - base) / denom;
     v3 lp = base + cn * t;
     v3 ref = closest_bary(pA, pB, pC, lp);
-    v3 sc = closest_on_edge(ref, posA, posB);
+    v3 sc = closest_on_edge(ref, k.posA, k.posB);
     v3 bary = closest_bary(pA, pB, pC, sc);
     v3 contact = pA * bary.x + pB * bary.y + pC * bary.z;
     v3 sv = sc - contact;

@@ -36,3 +36,25 @@ def test_joined_launches(gpu, oracle_lib, flags, tets, drag):
     x, want = m.vertex.cpu().numpy(), o.a["vertex"]
     assert np.abs(x - want).max() < POS_TOL * np.abs(want).max()
     assert np.abs(want - m.initialVertex.cpu().numpy()).max() > 1e-4  # it moved
+
+
+def test_contact_lanes(gpu):
+    # a triangle's four lanes (small models) and its one (from 100,000 triangles on) give the
+    # same responses: an env's contact on the positions as they are, alone and among its copies
+    mesh = mg.ellipsoid_for_tets(16000, seed=6)
+    out = []
+    for copies in (1, 33):
+        m, _ = sc.liver_model("cuda:0", copies, meshes=[mesh] * copies, substeps=1, iterations=1)
+        m.constraintFlags = L.COLLIDE
+        top = m.vertex[int(m.vertex[m.envSlice(0), 1].argmax())]  # the jaws' tips onto the surface
+        m.moveTool((top - m.laparoscopeTip[0]).repeat(copies, 1))
+        SimIntegratorDO("cuda:0", batched=False).stepModel(m, 1)
+        torch.cuda.synchronize()
+        for e in {0, copies - 1}:
+            out.append((int(m.laparoscopeInCollision[e]), m.vertex[m.envSlice(e)].cpu().numpy()))
+    assert len(mesh["triangle"]) < 100000 < 33 * len(mesh["triangle"])
+    assert out[0][0] > 0
+    for n, x in out[1:]:
+        assert n == out[0][0]
+        # sums of a few responses in any order: a few roundings of the position
+        np.testing.assert_allclose(x, out[0][1], rtol=0, atol=8 * np.finfo(np.float32).eps * np.abs(x).max())
