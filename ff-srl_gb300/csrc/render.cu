@@ -815,7 +815,8 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 // 256 envs of 500-20,000 tets at 128 x 128: a thread per ray took 1,224 us and 1,900
 // instructions a warp of 32 rays with two thirds of its lanes busy, the tiles 730; 8 textured
 // envs at 512 x 512: 540 and 275 us.  What bounds it now is issue, 65% of it, and on one env
-// the chain of loads, tests and shading of the tile with the most triangles (45 us).
+// the chain of loads, tests and shading of the patch with the most triangles (45 us with one
+// warp a patch, 35 with two: launch_rays).
 //
 // The hit is the traversal's: of the triangles whose test succeeds, the nearest, the first
 // in the reference's order among equals.  The traversal reaches a triangle if the ray's slab
@@ -829,6 +830,7 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 constexpr int kCand = 448;      // triangles of a tile, 64 bytes of shared memory each
 constexpr int kFront = 768;     // nodes of a level
 constexpr int kSteps = 40;
+constexpr int kTwoWarps = 608;  // the most tiles of 8 whose patches take two warps each
 constexpr int kList = 160;      // triangles a warp keeps for its four patches
 // Levels tested at once at the start.  Large images (T 16): at most 255 nodes, one a thread.
 // Small ones wait for each step more than for its work: at most 2,047 nodes, eight a thread.
@@ -844,8 +846,8 @@ __device__ __noinline__ Hit traverse(const ffsrl_render* r, const ffsrl_bvh* b, 
     return h;
 }
 
-template <int T>
-__global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_render r, const __grid_constant__ ffsrl_bvh b,
+template <int T, int HALVES>
+__global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_constant__ ffsrl_render r, const __grid_constant__ ffsrl_bvh b,
                                                  const int* __restrict__ ids, int n_ids) {
     __shared__ float4 s_tri[4 * kCand];  // (ab, ac, tvec, qvec, ac.qvec, leaf, place in the leaf, distance)
     __shared__ unsigned short s_list[T == 16 ? 8 : 1][kList];
@@ -853,12 +855,15 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
     __shared__ int s_leaf[kCand];
     __shared__ int s_n[3], s_leaves, s_over, s_nf, s_nb;
     __shared__ int s_todo[8][3];  // tiles still to do: x, y, size
+    __shared__ float s_hit[HALVES == 2 ? 8 : 1][3][HALVES == 2 ? 32 : 1];  // the second warp's rays: distance, second, triangle
+    constexpr int kThreads = 256 * HALVES;
     const int R = r.resolution, W = 2 * R, H = 2 * R;
     const int tiles_x = (R + T - 1) / T, tiles = tiles_x * tiles_x;
     const int k = blockIdx.x / tiles;
     const int e = ids ? (k < n_ids ? ids[k] : r.num_envs) : k;
     if (e < 0 || e >= r.num_envs) return;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = HALVES == 2 ? (tid >> 5) & 7 : tid >> 5;
+    const int part = HALVES == 2 ? tid >> 8 : 0;  // which of the patch's warps
     const int cam = r.num_cameras > 1 ? e : 0;
     const v3 ro = ld3(r.camera_pos, cam);
     const float4 qr = reinterpret_cast<const float4*>(r.camera_rot)[cam];
@@ -898,11 +903,11 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
                 const int topo = b.env_topology[e], lo = b.topo_level_offset[topo], deepest = b.topo_max_level[topo];
                 const int g = max(0, deepest - FirstLevel<T>::value);
                 const int s0 = b.level_start[lo + g], s1 = b.level_start[lo + g + 1], s2 = b.level_start[lo + deepest + 1];
-                for (int i0 = s0 + tid; i0 < s2; i0 += 1024) {
+                for (int i0 = s0 + tid; i0 < s2; i0 += 4 * kThreads) {
                     int node[4];  // four loads in flight
-                    for (int m = 0; m < 4; ++m) node[m] = i0 + 256 * m < s2 ? b.level_node[i0 + 256 * m] : -1;
+                    for (int m = 0; m < 4; ++m) node[m] = i0 + kThreads * m < s2 ? b.level_node[i0 + kThreads * m] : -1;
                     for (int m = 0; m < 4; ++m)
-                        if (i0 + 256 * m < s2) visit(node[m], &s_n[0], s_front[0], i0 + 256 * m < s1);
+                        if (i0 + kThreads * m < s2) visit(node[m], &s_n[0], s_front[0], i0 + kThreads * m < s1);
                 }
             } else if (tid == 0) {
                 visit(0, &s_n[0], s_front[0], true);
@@ -915,13 +920,13 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
                 const int n = min(s_n[step % 3], kFront);
                 if (n == 0 || step == kSteps) break;
                 if (tid == 0) s_n[(step + 2) % 3] = 0;
-                for (int i = tid; i < n; i += 256)
+                for (int i = tid; i < n; i += kThreads)
                     visit(s_front[step & 1][i], &s_n[(step + 1) % 3], s_front[(step + 1) & 1], true);
                 __syncthreads();
             }
             if (step == kSteps && tid == 0) s_over = 1;
             const int leaves = min(s_leaves, kCand);
-            for (int i = tid; i < leaves; i += 256) {
+            for (int i = tid; i < leaves; i += kThreads) {
                 const int node = s_leaf[i];
                 const float4 a = __ldg(ev.box + 2 * node), c = __ldg(ev.box + 2 * node + 1);
                 const int fc = __float_as_int(c.w), first = fc >> 8;
@@ -1020,15 +1025,8 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
                             const float ad = fabsf(det), su = det < 0.0f ? -nu : nu, sv = det < 0.0f ? -nv : nv;
                             return !(ad < 0.0001f || su < -1e-30f || sv < -1e-30f || su > 1.00001f * ad || su + sv > 1.00002f * ad);
                         };
-                        auto test = [&](int c, float det, float nu, float nv) {
-                            const float4 D = s_tri[4 * c + 3];
-                            const float invDet = 1.0f / det;
-                            const float u = nu * invDet;
-                            if (u < 0.0f || u > 1.0f) return;
-                            const float v = nv * invDet;
-                            if (v < 0.0f || u + v > 1.0f) return;
-                            const float t = D.x * invDet;
-                            if (!(t > 0.0f)) return;
+                        // a hit of triangle c at distance t
+                        auto take = [&](int c, float t, const float4& D) {
                             if (t > tMin) { second = fminf(second, t); return; }
                             second = tMin;
                             if (t == tMin) {  // the traversal keeps the first of equals in the reference's order
@@ -1040,9 +1038,20 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
                             tMin = t;
                             best = c;
                         };
+                        auto test = [&](int c, float det, float nu, float nv) {
+                            const float4 D = s_tri[4 * c + 3];
+                            const float invDet = 1.0f / det;
+                            const float u = nu * invDet;
+                            if (u < 0.0f || u > 1.0f) return;
+                            const float v = nv * invDet;
+                            if (v < 0.0f || u + v > 1.0f) return;
+                            const float t = D.x * invDet;
+                            if (!(t > 0.0f)) return;
+                            take(c, t, D);
+                        };
                         for (int side = 0; side < 2; ++side) {
                             const int c0 = !side ? 0 : own ? nf : kCand - nb, c1 = c0 + (side ? nb : nf);
-                            for (int cb = c0; cb < c1; cb += 32) {
+                            for (int cb = c0 + 32 * part; cb < c1; cb += 32 * HALVES) {
                                 // what lies behind every ray's hit so far is left out
                                 const float far = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(tMin)));
                                 int c = cb + lane;
@@ -1065,6 +1074,22 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
                                 }
                             }
                         }
+                        if constexpr (HALVES == 2) {
+                            // the first warp takes the second's hits as it would one triangle's
+                            if (part == 1) {
+                                s_hit[warp][0][lane] = tMin;
+                                s_hit[warp][1][lane] = second;
+                                s_hit[warp][2][lane] = __int_as_float(best);
+                            }
+                            asm volatile("bar.sync %0, 64;" ::"r"(1 + warp) : "memory");
+                            const float t = s_hit[warp][0][lane];
+                            const int other = __float_as_int(s_hit[warp][2][lane]);
+                            if (part == 0) {
+                                if (other >= 0) take(other, t, s_tri[4 * other + 3]);
+                                second = fminf(second, s_hit[warp][1][lane]);
+                            }
+                            asm volatile("bar.sync %0, 64;" ::"r"(1 + warp) : "memory");  // (read before the next tile's)
+                        }
                         if (best >= 0) {
                             const float4 D = s_tri[4 * best + 3];
                             const int leaf = __float_as_int(D.y);
@@ -1079,10 +1104,11 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
                             }
                         }
                     }
+                    if (HALVES == 2 && part == 1) continue;
                     if (walk) hit = traverse(&r, &b, e, ro, rd);
                     if (valid) s = shade(r, ev, e, hit.tri, hit.t, hit.p);
                 }
-                store_pixel(r, s, valid, e, px, py);
+                if (part == 0) store_pixel(r, s, valid, e, px, py);
             }
         }
         if (todo == 0) return;
@@ -1093,11 +1119,15 @@ __global__ void __launch_bounds__(256, 4) k_rays(const __grid_constant__ ffsrl_r
 }
 
 // Tiles of 16 pixels share the walk among 32 patches; tiles of 8, four times as many, where
-// those of 16 would give an SM fewer than seven
+// those of 16 would give an SM fewer than seven.  Where even those are few, the time is that of
+// the patch with the most triangles, some 70,000 cycles of tests on one warp: two warps share
+// its triangles (one env at 128 x 128, 256 tiles, 56 -> 46 us; two 56 -> 48; with four, 1,024
+// tiles, there is 3% in it, with fifteen it costs 10%).
 void launch_rays(const ffsrl_render& r, const ffsrl_bvh& b, const int32_t* ids, int n, cudaStream_t s) {
     auto tiles = [&](int t) { return ((long long)(r.resolution + t - 1) / t) * ((r.resolution + t - 1) / t) * n; };
-    if (tiles(16) >= 1024) k_rays<16><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n);
-    else k_rays<8><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
+    if (tiles(16) >= 1024) k_rays<16, 1><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n);
+    else if (tiles(8) <= kTwoWarps) k_rays<8, 2><<<(unsigned)tiles(8), 512, 0, s>>>(r, b, ids, n);
+    else k_rays<8, 1><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
 }
 
 int32_t check_bvh(const ffsrl_bvh* b) {

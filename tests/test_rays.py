@@ -47,7 +47,9 @@ def _camera(kind, meshes, seed):
     ("plain", 1, 1, "out", 4), ("plain", 2, 7, "out", 3), ("plain", 1, 33, "out", 1), ("plain", 3, 50, "near", 0),
     ("plain", 1, 128, "out", 2), ("dense", 1, 8, "out", 4), ("dense", 2, 16, "out", 4), ("dense", 1, 128, "near", 3),
     ("beam", 2, 64, "axis", 3), ("plain", 2, 64, "axis", 4), ("plain", 2, 48, "inside", 4), ("plain", 2, 40, "away", 4),
-    ("plain", 2, 40, "scaled", 4), ("plain", 70, 63, "out", 4), ("dense", 300, 17, "out", 4), ("beam", 18, 128, "axis", 4)])
+    ("plain", 2, 40, "scaled", 4), ("plain", 70, 63, "out", 4), ("dense", 300, 17, "out", 4), ("beam", 18, 128, "axis", 4),
+    # tiles of 8 whose patches have one warp each (more than 608, the cases above fewer)
+    ("plain", 3, 128, "out", 4), ("dense", 10, 64, "near", 3), ("beam", 3, 125, "axis", 4)])
 def test_tiles_give_the_traversal_s_depth(gpu, kind, envs, res, camera, mode):
     meshes = [_mesh(kind)] * envs
     m, _ = sc.liver_model("cuda:0", envs, meshes=meshes)
