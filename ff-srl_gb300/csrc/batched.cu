@@ -159,6 +159,14 @@ void free_batch(ffsrl_batch* b) {
 // either way; 800, reference, 12.3 and 14.0, 1,200 17.8 either way.  With the sums in global
 // scratch (mode 1) the 46,640-tet ellipsoid took 37.1 ms with 512 threads, 42.9 with 1,024.
 int few_envs(const ffsrl_batch* b) { return (b->arith == FFSRL_ARITH_FAST ? 6 : 7) * b->sm_count; }
+// Whether a class is short enough for large blocks, which run one to an SM, in a plan of few
+// envs: one wave of them, or three where an env has enough tets to keep 768 threads busy (300
+// envs of 304 vertices, reference: 837 us a step with three blocks of 256 to an SM, 909 with
+// 512 threads, 440 envs 1,077 and 1,354, 152 envs 630 and 468; of 904 vertices, 300 envs 2,641
+// and 2,486 with 768, 440 envs 3,546 and 3,716, 600 envs 4,814 and 4,955).
+bool few_members(const ffsrl_batch* b, int max_nv, size_t members) {
+    return members <= (size_t)(max_nv <= 512 ? 1 : 3) * b->sm_count;
+}
 int default_block(int max_nv, int mode, bool few) {
     if (mode == 2) return 256;
     if (mode == 1) return 512;
@@ -1511,7 +1519,7 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
         c.scratch_stride = plan_scratch(b, block_mode, c.max_nv);
         c.scratch_stride = (c.scratch_stride + 255) & ~(size_t)255;
         c.members = (int)mem.size();
-        int want = block_override > 0 ? block_override : default_block(c.max_nv, c.mode, N <= few_envs(b));
+        int want = block_override > 0 ? block_override : default_block(c.max_nv, c.mode, N <= few_envs(b) && few_members(b, c.max_nv, mem.size()));
         if (accum != FFSRL_ACC_FIXED && block_override <= 0 && c.max_nv <= 2560) want = std::min(want, 512);  // 768 are not built
         if (c.split > 1) {
             int items = 0;
