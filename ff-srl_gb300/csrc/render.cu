@@ -848,7 +848,7 @@ __device__ __noinline__ Hit traverse(const ffsrl_render* r, const ffsrl_bvh* b, 
 
 template <int T, int HALVES>
 __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_constant__ ffsrl_render r, const __grid_constant__ ffsrl_bvh b,
-                                                 const int* __restrict__ ids, int n_ids, bool alone) {
+                                                 const int* __restrict__ ids, int n_ids) {
     __shared__ float4 s_tri[4 * kCand];  // (ab, ac, tvec, qvec, ac.qvec, leaf, place in the leaf, distance)
     __shared__ unsigned short s_list[T == 16 ? 8 : 1][kList];
     __shared__ int s_front[2][kFront];
@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
     const float4 qr = reinterpret_cast<const float4*>(r.camera_rot)[cam];
     const EnvView ev = env_view(b, e);
     const Camera cm = make_camera(r, qr, W, H);
-    const bool packed = ev.box && ev.tpos && !alone;
+    const bool packed = ev.box && ev.tpos;
     int todo = 0;  // tiles in s_todo, the same for every thread
     int tx = ((blockIdx.x % tiles) % tiles_x) * T, ty = ((blockIdx.x % tiles) / tiles_x) * T, size = T;
     for (;;) {
@@ -1118,21 +1118,43 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
     }
 }
 
+// A thread per ray: a block traverses the rays of 8 x 8 pixels, a warp those of 4 x 2
+__global__ void __launch_bounds__(256) k_rays_alone(const __grid_constant__ ffsrl_render r, const __grid_constant__ ffsrl_bvh b,
+                                                    const int* __restrict__ ids, int n_ids) {
+    const int R = r.resolution, W = 2 * R, H = 2 * R;
+    const int tiles_x = (R + 7) / 8, tiles = tiles_x * tiles_x;
+    const int k = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+    const int e = ids ? (k < n_ids ? ids[k] : r.num_envs) : k;
+    const int warp = threadIdx.x >> 5, j = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+    const int px = (tile % tiles_x) * 8 + (warp & 1) * 4 + (j & 3), py = (tile / tiles_x) * 8 + (warp >> 1) * 2 + (j >> 2);
+    const bool valid = e >= 0 && e < r.num_envs && px < R && py < R;
+    Shade s;
+    s.color = mk(0.0f, 0.0f, 0.0f);
+    s.depth = 0.0f;
+    if (valid) {
+        const int cam = r.num_cameras > 1 ? e : 0;
+        const v3 ro = ld3(r.camera_pos, cam);
+        const float4 qr = reinterpret_cast<const float4*>(r.camera_rot)[cam];
+        const EnvView ev = env_view(b, e);
+        s = trace(r, ev, e, ro, qr, 2 * px + (q & 1), H - (2 * py + (q >> 1)), W, H);  // ray as in downsample_kernel
+    }
+    store_pixel(r, s, valid, e, px, py);
+}
+
 // Tiles of 16 pixels share the walk among 32 patches; tiles of 8, four times as many, where
 // those of 16 would give an SM fewer than seven.  Where even those are few, the time is that of
 // the patch with the most triangles, some 70,000 cycles of tests on one warp: two warps share
 // its triangles (one env at 128 x 128, 256 tiles, 56 -> 46 us; two 56 -> 48; with four, 1,024
 // tiles, there is 3% in it, with fifteen it costs 10%).
 // In small images a tile holds much of the mesh and its rays share little: each ray is
-// traversed alone (16 x 16, 1 and 216 envs: 44 and 109 us, by tiles 75 and 180; 50 x 50, 24 and
-// 216: 87 and 317, by tiles 127 and 331; 64 x 64, 24 envs 97 and 139, 216 424 and 349).
+// traversed alone (16 x 16, 1 and 216 envs: 43 and 91 us, by tiles 75 and 180; 50 x 50, 24 and
+// 216: 75 and 235, by tiles 127 and 331; 64 x 64, 24 and 216: 81 and 317, by tiles 139 and 349).
 void launch_rays(const ffsrl_render& r, const ffsrl_bvh& b, const int32_t* ids, int n, cudaStream_t s) {
     auto tiles = [&](int t) { return ((long long)(r.resolution + t - 1) / t) * ((r.resolution + t - 1) / t) * n; };
-    const bool alone = r.resolution <= 50 || (r.resolution <= 64 && n <= 64);
-    if (alone) k_rays<8, 1><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n, true);
-    else if (tiles(16) >= 1024) k_rays<16, 1><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n, false);
-    else if (tiles(8) <= kTwoWarps) k_rays<8, 2><<<(unsigned)tiles(8), 512, 0, s>>>(r, b, ids, n, false);
-    else k_rays<8, 1><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n, false);
+    if (r.resolution <= 64) k_rays_alone<<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
+    else if (tiles(16) >= 1024) k_rays<16, 1><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n);
+    else if (tiles(8) <= kTwoWarps) k_rays<8, 2><<<(unsigned)tiles(8), 512, 0, s>>>(r, b, ids, n);
+    else k_rays<8, 1><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
 }
 
 int32_t check_bvh(const ffsrl_bvh* b) {
