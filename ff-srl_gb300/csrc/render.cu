@@ -1148,10 +1148,14 @@ __global__ void __launch_bounds__(256) k_rays_alone(const __grid_constant__ ffsr
 // tiles, there is 3% in it, with fifteen it costs 10%).
 // In small images a tile holds much of the mesh and its rays share little: each ray is
 // traversed alone (16 x 16, 1 and 216 envs: 43 and 91 us, by tiles 75 and 180; 50 x 50, 24 and
-// 216: 75 and 235, by tiles 127 and 331; 64 x 64, 24 and 216: 81 and 317, by tiles 139 and 349).
+// 216: 75 and 235, by tiles 127 and 331; 64 x 64, 24 and 216: 81 and 317, by tiles 139 and 349).  So
+// are images of up to 128 pixels where the tiles are too few to hide one another's chains (24
+// envs of 500-15,000 tets, 80, 100 and 128 pixels: 96, 120 and 154 us, by tiles 162, 177 and 174;
+// 216 envs at 128: 1,007 and 710; one env at 128: 70 and 43).
 void launch_rays(const ffsrl_render& r, const ffsrl_bvh& b, const int32_t* ids, int n, cudaStream_t s) {
     auto tiles = [&](int t) { return ((long long)(r.resolution + t - 1) / t) * ((r.resolution + t - 1) / t) * n; };
-    if (r.resolution <= 64) k_rays_alone<<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
+    if (r.resolution <= 64 || (r.resolution <= 128 && tiles(8) > kTwoWarps && tiles(16) < 1600))
+        k_rays_alone<<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
     else if (tiles(16) >= 1024) k_rays<16, 1><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n);
     else if (tiles(8) <= kTwoWarps) k_rays<8, 2><<<(unsigned)tiles(8), 512, 0, s>>>(r, b, ids, n);
     else k_rays<8, 1><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
