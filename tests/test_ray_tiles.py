@@ -1,0 +1,153 @@
+"""The ray-cast by tiles (images above 64 pixels, but for mid-sized batches of up to 128)
+against the reference-shaped renderer, which traverses every ray: the same depth bit for bit
+from each of its three kernels -- tiles of 16 (many pixels), tiles of 8, and tiles of 8 with
+two warps a patch (few pixels) -- for every kind of camera, where a tile has more triangles
+than its list (quarters, rays traversed one by one), without the arrays that the ray-cast can
+do without, and on a tree deeper than the traversal's stack."""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import test_render_overflow
+from ffsrl import SimBVH, WarpRaycastRendererDO, _lib as L, meshgen as mg, scenarios as sc
+
+pytestmark = pytest.mark.gpu
+
+_MESHES = {}
+
+
+def _kernel(envs, res):
+    """The kernel that images of this size take (the rule of the dispatch)."""
+    tiles = [envs * (-(-res // t)) ** 2 for t in (8, 16)]
+    if res <= 64 or (res <= 128 and tiles[0] > 608 and tiles[1] < 1600):
+        return "rays"
+    return "16" if tiles[1] >= 1024 else "8x2" if tiles[0] <= 608 else "8"
+
+
+def _mesh(kind):
+    if kind not in _MESHES:
+        if kind == "dense":
+            m = mg.ellipsoid()
+        elif kind == "textured":
+            m = mg.add_texture(mg.ellipsoid_for_tets(1500), size=64, seed=1)
+        else:
+            m = mg.beam(jitter=0.0) if kind == "beam" else mg.ellipsoid_for_tets(1500)
+            lo, hi = m["vertex"].min(axis=0) - 2.0, m["vertex"].max(axis=0) + 2.0
+            m = mg.with_rigids(m, [mg.rigid_box([lo[0], lo[1] - 0.5, lo[2]], [hi[0], lo[1], hi[2]])])
+        _MESHES[kind] = m
+    return _MESHES[kind]
+
+
+def _camera(kind, meshes, seed):
+    pos, rot = sc.env_cameras(meshes, seed=seed)
+    c = np.stack([m["vertex"].mean(axis=0) for m in meshes])
+    if kind == "inside":
+        pos = c.astype(np.float32)
+    elif kind == "away":
+        pos = (2.0 * pos - c).astype(np.float32) + 40.0
+    elif kind == "axis":  # straight along -z from a point level with the mesh's vertices
+        pos = np.round(c).astype(np.float32) + np.float32([0.0, 0.0, 30.0])
+        rot = np.tile(np.float32([0.0, 0.0, 0.0, 1.0]), (len(meshes), 1))
+    elif kind == "scaled":
+        rot = (rot * 1.1).astype(np.float32)
+    elif kind == "near":
+        pos = (c + 0.4 * (pos - c)).astype(np.float32)
+    return pos, rot
+
+
+def _compare(m, bvh, meshes, envs, res, camera, mode, seed):
+    ap = sc.fov_aperture(60.0)
+    out = []
+    for fused in (False, True):
+        r = WarpRaycastRendererDO("cuda:0", m, resolution=res, mode="headless", verticalAperture=ap,
+                                  horizontalAperture=ap, fused=fused, render_mode=mode)
+        r.setCameras(*_camera(camera, meshes, seed=seed))
+        r.depth.fill_(-1.0)
+        r.pixels.fill_(-1.0)
+        r.renderNew(bvh, m)
+        torch.cuda.synchronize()
+        r.checkErrors()
+        out.append(r)
+    a, b = (r.depthImages().cpu().numpy() for r in out)
+    assert np.array_equal(a, b), f"{(a != b).sum()} of {a.size} depths differ"
+    assert (a == 0.0).all() if camera == "away" else (a > 0.0).any()
+    # (the two sum the vertex normals in different orders)
+    np.testing.assert_allclose(out[1].pixels.cpu().numpy(), out[0].pixels.cpu().numpy(), atol=2e-4)
+    # a list of envs writes theirs alone
+    r = out[1]
+    ids = torch.tensor([envs - 1], dtype=torch.int32, device="cuda:0")
+    r.depth.fill_(-1.0)
+    L.check(L.lib().ffsrl_render_fused_envs(C.byref(r._desc(m)), C.byref(bvh.desc), L.ptr(ids), 1, None))
+    got = r.depthImages().cpu().numpy()
+    np.testing.assert_array_equal(got[envs - 1], b[envs - 1])
+    assert envs == 1 or (got[:envs - 1] == -1.0).all()
+
+
+@pytest.mark.parametrize("kernel,kind,envs,res,camera,mode", [
+    ("8x2", "plain", 1, 70, "out", 1), ("8x2", "plain", 2, 101, "axis", 4), ("8x2", "beam", 1, 128, "axis", 4),
+    ("8x2", "dense", 1, 128, "out", 4), ("8x2", "plain", 2, 96, "inside", 4), ("8x2", "plain", 1, 80, "away", 4),
+    ("8x2", "plain", 2, 88, "scaled", 2), ("8x2", "dense", 1, 150, "near", 3), ("8x2", "textured", 1, 128, "near", 1),
+    ("8", "plain", 1, 205, "out", 3), ("8", "beam", 2, 150, "axis", 4), ("8", "dense", 3, 140, "out", 4),
+    ("8", "plain", 2, 192, "inside", 4), ("8", "plain", 2, 160, "away", 4), ("8", "plain", 3, 131, "scaled", 4),
+    ("8", "dense", 1, 256, "near", 0), ("8", "textured", 2, 200, "out", 1),
+    ("16", "plain", 1, 512, "out", 1), ("16", "plain", 30, 128, "out", 3), ("16", "beam", 30, 125, "axis", 4),
+    ("16", "dense", 2, 400, "near", 4), ("16", "dense", 100, 66, "out", 4), ("16", "plain", 2, 515, "inside", 4),
+    ("16", "plain", 4, 260, "away", 4), ("16", "plain", 4, 270, "scaled", 4), ("16", "textured", 2, 512, "near", 1)])
+def test_each_kernel(gpu, kernel, kind, envs, res, camera, mode):
+    assert _kernel(envs, res) == kernel
+    meshes = [_mesh(kind)] * envs
+    m, _ = sc.liver_model("cuda:0", envs, meshes=meshes)
+    _compare(m, SimBVH("cuda:0", m), meshes, envs, res, camera, mode, res)
+
+
+@pytest.mark.parametrize("kernel,envs,res", [("8x2", 2, 100), ("8", 2, 180), ("16", 2, 400)])
+@pytest.mark.parametrize("without", ["packed copies", "level lists"])
+def test_optional_arrays_left_out(gpu, kernel, envs, res, without):
+    assert _kernel(envs, res) == kernel
+    meshes = [_mesh("plain")] * envs
+    m, _ = sc.liver_model("cuda:0", envs, meshes=meshes)
+    bvh = SimBVH("cuda:0", m)
+    r = WarpRaycastRendererDO("cuda:0", m, resolution=res, mode="headless")
+    r.setCameras(*_camera("out", meshes, seed=3))
+    r.renderNew(bvh, m)
+    want = r.depthImages().cpu().numpy().copy()
+    if without == "packed copies":
+        bvh.desc.node_box = bvh.desc.tri_pos = None
+    else:
+        bvh.desc.level_node = bvh.desc.level_start = bvh.desc.topo_level_offset = None
+    r.depth.zero_()
+    r.renderNew(bvh, m)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(r.depthImages().cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("kernel,envs,res", [("8x2", 1, 128), ("8", 2, 180), ("16", 2, 400)])
+def test_depth_equals_the_oracle_s(gpu, oracle_lib, kernel, envs, res):
+    assert _kernel(envs, res) == kernel
+    meshes = [_mesh("plain")] * envs
+    m, _ = sc.liver_model("cuda:0", envs, meshes=meshes)
+    bvh = SimBVH("cuda:0", m)
+    r = WarpRaycastRendererDO("cuda:0", m, resolution=res, mode="headless", render_mode=3)
+    r.setCameras(*_camera("out", meshes, seed=7))
+    r.renderNew(bvh, m)
+    torch.cuda.synchronize()
+    color, depth, _ = oracle_lib.render(r, bvh, m.allVisPoint.cpu().numpy())
+    np.testing.assert_array_equal(r.depthImages().cpu().numpy(), depth)
+    np.testing.assert_allclose(r.pixels.view(color.shape).cpu().numpy(), color, atol=2e-4)
+
+
+@pytest.mark.parametrize("kernel,res", [("8x2", 100), ("8", 200), ("16", 512)])
+def test_overflow_is_reported(gpu, kernel, res):
+    assert _kernel(1, res) == kernel
+    m = test_render_overflow._model("cuda:0")
+    bvh = SimBVH("cuda:0", m)
+    r = WarpRaycastRendererDO("cuda:0", m, resolution=res, mode="headless", render_mode=4)
+    r.setCameras(*test_render_overflow._camera())
+    r.renderNew(bvh, m)
+    torch.cuda.synchronize()
+    with pytest.raises(L.FFSRLError) as e:
+        r.checkErrors()
+    assert e.value.code == L.ERR_STACK_OVERFLOW
