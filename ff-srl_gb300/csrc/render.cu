@@ -730,41 +730,64 @@ __device__ __forceinline__ Camera make_camera(const ffsrl_render& r, float4 q, i
     c.dy = quat_rotate(q, mk(0.0f, 2.0f * ty / float(H), 0.0f));
     return c;
 }
-// The four corners of a rectangle of w x h pixels' rays from pixel (px, py), widened by a
-// quarter of the ray spacing on each side: far more than rounding moves a ray's direction
-// (some 3e-7), so every ray of the rectangle lies between the corners
+// The rays of a rectangle of w x h pixels from pixel (px, py), as ranges of the ray indices
+// widened by a quarter of the ray spacing on each side
+struct Range { float x0, x1, y0, y1; };
+__device__ __forceinline__ Range ray_range(int px, int py, int w, int h, int H) {
+    return {2.0f * px - 0.25f, 2.0f * (px + w) - 0.75f, H - (2.0f * (py + h) - 0.75f), H - (2.0f * py - 0.25f)};
+}
+// The four corners of the rectangle: every ray of it lies between them, to within the rounding
+// of a direction (some 1e-6 of it; of the outermost corner through very wide lenses)
 struct Corners { v3 d[4]; };
 __device__ __forceinline__ Corners make_corners(const Camera& c, int px, int py, int w, int h, int H) {
-    const float x0 = 2.0f * px - 0.25f, x1 = 2.0f * (px + w) - 0.75f;
-    const float y0 = H - (2.0f * (py + h) - 0.75f), y1 = H - (2.0f * py - 0.25f);
-    const v3 a = c.d0 + x0 * c.dx, b = c.d0 + x1 * c.dx;
+    const Range g = ray_range(px, py, w, h, H);
+    const v3 a = c.d0 + g.x0 * c.dx, b = c.d0 + g.x1 * c.dx;
     Corners k;
-    k.d[0] = a + y0 * c.dy; k.d[1] = b + y0 * c.dy; k.d[2] = b + y1 * c.dy; k.d[3] = a + y1 * c.dy;
+    k.d[0] = a + g.y0 * c.dy; k.d[1] = b + g.y0 * c.dy; k.d[2] = b + g.y1 * c.dy; k.d[3] = a + g.y1 * c.dy;
     return k;
 }
-// The planes through the camera between them, normals inward; outside() leaves a relative
-// 2e-6 on top, as the slab test sees a box's edges with that much rounding.  (A zero or
-// non-finite normal excludes nothing.)
+// The camera's axes, z into the picture: what quat_rotate makes of (1, 0, 0), (0, 1, 0) and
+// (0, 0, -1)
+struct Axes { v3 x, y, z; };
+__device__ __forceinline__ Axes make_axes(float4 q) {
+    const float c = 2.0f * q.w * q.w - 1.0f;
+    Axes a;
+    a.x = mk(c + 2.0f * q.x * q.x, 2.0f * (q.x * q.y + q.w * q.z), 2.0f * (q.x * q.z - q.w * q.y));
+    a.y = mk(2.0f * (q.x * q.y - q.w * q.z), c + 2.0f * q.y * q.y, 2.0f * (q.y * q.z + q.w * q.x));
+    a.z = mk(-2.0f * (q.x * q.z + q.w * q.y), -2.0f * (q.y * q.z - q.w * q.x), -(c + 2.0f * q.z * q.z));
+    return a;
+}
+__device__ __forceinline__ float sum1(v3 a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
+// A quaternion far from a unit one can make the axes shrink to rounding errors, or nearly
+// parallel.  The margins here hold while their volume is not far below that of a rotation's.
+__device__ __forceinline__ bool sound(const Axes& a, float4 q) {
+    const float n = 1.0f + 2.0f * (q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
+    return fabsf(dot(cross(a.x, a.y), a.z)) > 0.02f * n * n * n;
+}
+// The planes through the camera along a rectangle's sides, normals inward.  A side's normal is
+// the product of a direction on it and the camera's axis along it, z + e x and y, or z + e y and
+// x: perpendicular vectors, whereas two corners of a tile are nearly parallel behind a narrow
+// lens, and the rounding of their product then moves the plane by more than any margin (tiles of
+// 8 at 1,024 pixels: through a 5 degree lens 6% of the points on their outermost rays lay outside
+// their planes).  Rounding moves a normal by some 1e-6 of it, a ray's direction and the edges of a
+// box that the slab test sees by less; outside() leaves a relative 4e-6.  (A normal that is not
+// finite excludes nothing.)
 struct Bundle { v3 n[4]; };
-__device__ __forceinline__ Bundle make_bundle(const Corners& k) {
-    const v3 c = (k.d[0] + k.d[2]) + (k.d[1] + k.d[3]);
-    Bundle b;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const v3 n = cross(k.d[i], k.d[(i + 1) & 3]);
-        const float m = fabsf(n.x) + fabsf(n.y) + fabsf(n.z);
-        const float f = __fdividef(dot(n, c) < 0.0f ? -1.0f : 1.0f, m);
-        b.n[i] = m > 0.0f ? n * f : mk(0.0f, 0.0f, 0.0f);
-    }
-    return b;
+// side i: left, right, lower, upper
+__device__ __forceinline__ v3 make_plane(const Axes& c, const Range& g, float tx, float ty, int W, int H, int i) {
+    const bool across = i < 2;
+    const float t = across ? tx : ty, per = __fdividef(2.0f * t, float(across ? W : H));
+    const float e0 = per * (across ? g.x0 : g.y0) - t, e1 = per * (across ? g.x1 : g.y1) - t;
+    const v3 xy = cross(c.x, c.y), u = cross(across ? c.z : c.x, across ? c.y : c.z);
+    const v3 n = u + (i & 1 ? fmaxf(e0, e1) : fminf(e0, e1)) * xy;
+    const float s = (dot(xy, c.z) < 0.0f) == !(i & 1) ? 1.0f : -1.0f;  // (a quaternion may make a mirror image)
+    return n * __fdividef(s, sum1(n));
 }
 
 __device__ __forceinline__ float fdot(v3 a, v3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
 __device__ __forceinline__ v3 fcross(v3 a, v3 b) {
     return mk(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
 }
-__device__ __forceinline__ float sum1(v3 a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
-
 // Whether a ray between the corners can pass the triangle test: its determinant and the
 // numerators of u and v are linear in the direction, so where the determinant has one sign
 // at all corners, and u, v or 1 - u - v the wrong one, by more than the test's own rounding
@@ -792,7 +815,7 @@ __device__ __forceinline__ bool may_hit(const Corners& k, v3 ab, v3 ac, v3 tv, v
 __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
     const v3 c = mk(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
     const v3 h = mk(0.5f * (hi.x - lo.x), 0.5f * (hi.y - lo.y), 0.5f * (hi.z - lo.z));
-    const float g = 2e-6f * ((fabsf(c.x) + fabsf(c.y)) + (fabsf(c.z) + h.x) + (h.y + h.z));
+    const float g = 4e-6f * ((fabsf(c.x) + fabsf(c.y)) + (fabsf(c.z) + h.x) + (h.y + h.z));
     bool out = false;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -853,6 +876,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
     __shared__ unsigned short s_list[T == 16 ? 8 : 1][kList];
     __shared__ int s_front[2][kFront];
     __shared__ int s_leaf[kCand];
+    __shared__ float4 s_plane[4];  // the tile's bundle
     __shared__ int s_n[3], s_leaves, s_over, s_nf, s_nb;
     __shared__ int s_todo[8][3];  // tiles still to do: x, y, size
     __shared__ float s_hit[HALVES == 2 ? 8 : 1][3][HALVES == 2 ? 32 : 1];  // the second warp's rays: distance, second, triangle
@@ -874,10 +898,18 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
     int tx = ((blockIdx.x % tiles) % tiles_x) * T, ty = ((blockIdx.x % tiles) / tiles_x) * T, size = T;
     for (;;) {
         if (tid < 3) s_n[tid] = 0;
-        if (tid == 0) { s_leaves = 0; s_over = 0; s_nf = 0; s_nb = 0; }
+        if (tid == 0) { s_leaves = 0; s_nf = 0; s_nb = 0; }
+        if (tid < 4) {
+            const Axes axes = make_axes(qr);
+            const v3 n = make_plane(axes, ray_range(tx, ty, size, size, H), r.camera_tan * r.camera_aspect, r.camera_tan, W, H, tid);
+            s_plane[tid] = make_float4(n.x, n.y, n.z, 0.0f);
+            if (tid == 0) s_over = !sound(axes, qr);  // (then every ray is traversed)
+        }
         __syncthreads();
         if (packed) {
-            const Bundle F = make_bundle(make_corners(cm, tx, ty, size, size, H));
+            Bundle F;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) F.n[i] = mk(s_plane[i].x, s_plane[i].y, s_plane[i].z);
             auto visit = [&](int node, int* count, int* front, bool expand) {
                 if ((unsigned)node >= (unsigned)ev.nn) { s_over = 1; return; }
                 const float4 a = __ldg(ev.box + 2 * node), c = __ldg(ev.box + 2 * node + 1);

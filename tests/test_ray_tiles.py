@@ -2,8 +2,8 @@
 against the reference-shaped renderer, which traverses every ray: the same depth bit for bit
 from each of its three kernels -- tiles of 16 (many pixels), tiles of 8, and tiles of 8 with
 two warps a patch (few pixels) -- for every kind of camera, where a tile has more triangles
-than its list (quarters, rays traversed one by one), without the arrays that the ray-cast can
-do without, and on a tree deeper than the traversal's stack."""
+than its list (quarters, rays traversed one by one), behind narrow lenses, without the arrays
+that the ray-cast can do without, and on a tree deeper than the traversal's stack."""
 
 import ctypes as C
 
@@ -12,7 +12,7 @@ import pytest
 import torch
 
 import test_render_overflow
-from ffsrl import SimBVH, WarpRaycastRendererDO, _lib as L, meshgen as mg, scenarios as sc
+from ffsrl import SimBVH, SimModelDO, WarpRaycastRendererDO, _lib as L, meshgen as mg, scenarios as sc
 
 pytestmark = pytest.mark.gpu
 
@@ -101,6 +101,51 @@ def test_each_kernel(gpu, kernel, kind, envs, res, camera, mode):
     meshes = [_mesh(kind)] * envs
     m, _ = sc.liver_model("cuda:0", envs, meshes=meshes)
     _compare(m, SimBVH("cuda:0", m), meshes, envs, res, camera, mode, res)
+
+
+def _triangles(v, envs=1):
+    """A model of separate triangles v [n, 3, 3] and its BVH."""
+    mesh = mg.tiny_mesh(np.asarray(v, np.float32).reshape(-1, 3), triangle=np.arange(3 * len(v)).reshape(-1, 3))
+    m = SimModelDO(mesh, envs, "cuda:0")
+    return m, SimBVH("cuda:0", m)
+
+
+def _differ(m, bvh, res, fov, pos, rot, mode):
+    """Pixels whose depth or colour the two renderers give differently, and pixels with a hit
+    (no two triangles share a point, so that no normal is a sum)."""
+    images = []
+    for fused in (False, True):
+        r = WarpRaycastRendererDO("cuda:0", m, resolution=res, mode="headless", verticalAperture=sc.fov_aperture(fov),
+                                  horizontalAperture=sc.fov_aperture(fov), fused=fused, render_mode=mode)
+        r.setCameras(pos, rot)
+        r.renderNew(bvh, m)
+        torch.cuda.synchronize()
+        r.checkErrors()
+        images.append(torch.cat([r.pixels, r.depth[:, None]], dim=1).cpu().numpy())
+    return int((images[0] != images[1]).any(axis=1).sum()), int((images[0][:, 3] > 0.0).sum())
+
+
+@pytest.mark.parametrize("kernel,fov,res", [("8x2", 0.2, 128), ("8", 0.2, 256), ("8", 0.5, 480), ("16", 0.5, 1024),
+                                            ("16", 1.0, 1024), ("16", 2.0, 1024), ("16", 5.0, 1024)])
+@pytest.mark.parametrize("size", [1.0, 1.1])
+def test_narrow_lenses(gpu, kernel, fov, res, size):
+    # the sides of a tile are as little as some 1e-4 radians apart: triangles of a few rays'
+    # width, so that many reach just across a side.  (Below 1e-2 a side a triangle's determinant
+    # is under the test's limit, whatever the ray.)  size: of the camera's quaternion
+    assert _kernel(1, res) == kernel
+    for seed in range(4):
+        rng = np.random.Generator(np.random.PCG64(seed))
+        n, t = max(300, int(4e-3 * res * res)), np.tan(np.radians(fov) / 2.0)
+        width = np.exp(rng.uniform(np.log(2.0), np.log(12.0), n)) * t / res
+        far = np.maximum(20.0, 0.03 / width) * rng.uniform(1.0, 3.0, n)
+        d = np.stack([rng.uniform(-t, t, n), rng.uniform(-t, t, n), np.full(n, -1.0)], axis=1) * far[:, None]
+        q = rng.normal(size=4)
+        q *= size / np.linalg.norm(q)
+        u, w = q[:3], q[3]
+        c = d * (2.0 * w * w - 1.0) + 2.0 * (d @ u)[:, None] * u + 2.0 * w * np.cross(u, d)
+        m, bvh = _triangles(c[:, None, :] + rng.normal(size=(n, 3, 3)) * (width * far)[:, None, None])
+        differ, hit = _differ(m, bvh, res, fov, np.zeros((1, 3)), q[None], 2)
+        assert differ == 0 and hit > 300, f"seed {seed}: {differ} pixels differ, {hit} are hit"
 
 
 @pytest.mark.parametrize("kernel,envs,res", [("8x2", 2, 100), ("8", 2, 180), ("16", 2, 400)])
