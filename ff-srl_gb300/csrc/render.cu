@@ -844,12 +844,12 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 // The hit is the traversal's: of the triangles whose test succeeds, the nearest, the first
 // in the reference's order among equals.  The traversal reaches a triangle if the ray's slab
 // test enters its leaf's box (it then enters the boxes above, as rounding is monotone) and
-// no hit before it is nearer than that entry, so the nearest one's leaf is put to the slab
-// test at the end.  In the rare case that the test fails, or puts the entry behind another
-// hit (two triangles hit in a box's corner, where the one that is kept hangs on the order of
-// the traversal), the ray is traversed.  So is a ray along a coordinate plane, and every ray
-// of a 4 x 4 tile that still has too many triangles, or of a tree deeper than kSteps levels
-// below the ones tested first.
+// every hit before it is farther than that entry, so the nearest one's leaf is put to the slab
+// test at the end.  In the rare case that the test fails, or puts the entry no nearer than another
+// hit (two triangles hit in a box's corner, or at the same distance in a plane that bounds their
+// boxes, where the one that is kept hangs on the order of the traversal), the ray is traversed.
+// So is a ray along a coordinate plane, and every ray of a 4 x 4 tile that still has too many
+// triangles, or of a tree deeper than kSteps levels below the ones tested first.
 constexpr int kCand = 448;      // triangles of a tile, 64 bytes of shared memory each
 constexpr int kFront = 768;     // nodes of a level
 constexpr int kSteps = 40;
@@ -1127,7 +1127,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                             const int leaf = __float_as_int(D.y);
                             const float4 a = __ldg(ev.box + 2 * leaf), c = __ldg(ev.box + 2 * leaf + 1);
                             float tn;
-                            if (slab(ro, rd, mk(a.x, a.y, a.z), mk(c.x, c.y, c.z), tn) && (tn <= tMin || tn < second)) {
+                            if (slab(ro, rd, mk(a.x, a.y, a.z), mk(c.x, c.y, c.z), tn) && tn < second) {
                                 hit.t = tMin;
                                 hit.p = ro + tMin * rd;
                                 hit.tri = (int)(ev.fofs + ev.tri[ev.first[leaf] + __float_as_int(D.z)]);

@@ -2,8 +2,9 @@
 against the reference-shaped renderer, which traverses every ray: the same depth bit for bit
 from each of its three kernels -- tiles of 16 (many pixels), tiles of 8, and tiles of 8 with
 two warps a patch (few pixels) -- for every kind of camera, where a tile has more triangles
-than its list (quarters, rays traversed one by one), behind narrow lenses, without the arrays
-that the ray-cast can do without, and on a tree deeper than the traversal's stack."""
+than its list (quarters, rays traversed one by one), behind narrow lenses, where triangles
+are hit at the same distance, without the arrays that the ray-cast can do without, and on a
+tree deeper than the traversal's stack."""
 
 import ctypes as C
 
@@ -146,6 +147,26 @@ def test_narrow_lenses(gpu, kernel, fov, res, size):
         m, bvh = _triangles(c[:, None, :] + rng.normal(size=(n, 3, 3)) * (width * far)[:, None, None])
         differ, hit = _differ(m, bvh, res, fov, np.zeros((1, 3)), q[None], 2)
         assert differ == 0 and hit > 300, f"seed {seed}: {differ} pixels differ, {hit} are hit"
+
+
+@pytest.mark.parametrize("kernel,res", [("8x2", 128), ("8", 200), ("16", 512)])
+def test_equally_near_triangles(gpu, kernel, res):
+    # plates in coordinate planes, on a coarse grid: many rays hit two of them at the same
+    # distance, which is that of their boxes, too; the normals tell which one was kept
+    assert _kernel(1, res) == kernel
+    for seed in range(6):
+        rng = np.random.Generator(np.random.PCG64(seed))
+        v = []
+        for _ in range(600):
+            c = np.array([*(rng.integers(-12, 13, 2) / 2.0), rng.integers(-30, -9)])
+            across = rng.permutation(3)[:2]
+            b, d = c.copy(), c.copy()
+            b[across[0]] += rng.choice([0.5, 1.0, 2.0]) * rng.choice([-1, 1])
+            d[across[1]] += rng.choice([0.5, 1.0, 2.0]) * rng.choice([-1, 1])
+            v.append([c, b, d])
+        m, bvh = _triangles(v)
+        differ, hit = _differ(m, bvh, res, 60.0, np.zeros((1, 3)), np.array([[0.0, 0.0, 0.0, 1.0]]), 2)
+        assert differ == 0 and hit > 1000, f"seed {seed}: {differ} pixels differ, {hit} are hit"
 
 
 @pytest.mark.parametrize("kernel,envs,res", [("8x2", 2, 100), ("8", 2, 180), ("16", 2, 400)])
