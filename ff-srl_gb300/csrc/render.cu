@@ -876,7 +876,8 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
     __shared__ unsigned short s_list[T == 16 ? 8 : 1][kList];
     __shared__ int s_front[2][kFront];
     __shared__ int s_leaf[kCand];
-    __shared__ float4 s_plane[4];  // the tile's bundle
+    // the tile's planes; its middle ray and the longest ray's length, half its width and height
+    __shared__ float4 s_plane[7];
     __shared__ int s_n[3], s_leaves, s_over, s_nf, s_nb;
     __shared__ int s_todo[8][3];  // tiles still to do: x, y, size
     __shared__ float s_hit[HALVES == 2 ? 8 : 1][3][HALVES == 2 ? 32 : 1];  // the second warp's rays: distance, second, triangle
@@ -905,11 +906,20 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
             s_plane[tid] = make_float4(n.x, n.y, n.z, 0.0f);
             if (tid == 0) s_over = !sound(axes, qr);  // (then every ray is traversed)
         }
+        if (tid == 32) {
+            const Range g = ray_range(tx, ty, size, size, H);
+            const v3 mid = cm.d0 + 0.5f * (g.x0 + g.x1) * cm.dx + 0.5f * (g.y0 + g.y1) * cm.dy;
+            const v3 across = 0.5f * (g.x1 - g.x0) * cm.dx, up = 0.5f * (g.y1 - g.y0) * cm.dy;
+            s_plane[4] = make_float4(mid.x, mid.y, mid.z, sum1(mid) + sum1(across) + sum1(up));
+            s_plane[5] = make_float4(across.x, across.y, across.z, 0.0f);
+            s_plane[6] = make_float4(up.x, up.y, up.z, 0.0f);
+        }
         __syncthreads();
         if (packed) {
+            auto plane = [&](int i) { return mk(s_plane[i].x, s_plane[i].y, s_plane[i].z); };
             Bundle F;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) F.n[i] = mk(s_plane[i].x, s_plane[i].y, s_plane[i].z);
+            for (int i = 0; i < 4; ++i) F.n[i] = plane(i);
             auto visit = [&](int node, int* count, int* front, bool expand) {
                 if ((unsigned)node >= (unsigned)ev.nn) { s_over = 1; return; }
                 const float4 a = __ldg(ev.box + 2 * node), c = __ldg(ev.box + 2 * node + 1);
@@ -960,14 +970,9 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
             const int leaves = min(s_leaves, kCand);
             for (int i = tid; i < leaves; i += kThreads) {
                 const int node = s_leaf[i];
-                const float4 a = __ldg(ev.box + 2 * node), c = __ldg(ev.box + 2 * node + 1);
-                const int fc = __float_as_int(c.w), first = fc >> 8;
+                const int fc = __float_as_int(__ldg(ev.box + 2 * node + 1).w), first = fc >> 8;
                 int cnt = fc & 255;
                 if (cnt == 255) cnt = ev.count[node];
-                // distance of the box, a little less: no ray hits in it nearer than that
-                const v3 lo = mk(a.x, a.y, a.z) - ro, hi = mk(c.x, c.y, c.z) - ro;
-                const v3 gap = mk(fmaxf(fmaxf(lo.x, -hi.x), 0.0f), fmaxf(fmaxf(lo.y, -hi.y), 0.0f), fmaxf(fmaxf(lo.z, -hi.z), 0.0f));
-                const float near = length(gap) * 0.9999f;
                 for (int m = 0; m < cnt; ++m) {
                     const float4* q = ev.tpos + 3ll * (first + m);
                     const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
@@ -976,6 +981,17 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                     const float tn = dot(ac, qv);
                     const int at = tn > 0.0f ? atomicAdd(&s_nf, 1) : kCand - 1 - atomicAdd(&s_nb, 1);
                     if ((unsigned)at >= (unsigned)kCand) continue;  // too many: counted below
+                    // No ray finds a hit of it nearer than its own box lies (its leaf's box may be
+                    // another face's), less what rounding can do to a distance: some 32 units in
+                    // the last place of |ab| |ac| (|tv| + |ab| + |ac|) over the determinant, which
+                    // is 1e-4 at least, and much more where no ray of the tile grazes the triangle
+                    const v3 lo = vmin(vmin(ab, ac), mk(0.0f, 0.0f, 0.0f)) - tv, hi = vmax(vmax(ab, ac), mk(0.0f, 0.0f, 0.0f)) - tv;
+                    const v3 gap = mk(fmaxf(fmaxf(lo.x, -hi.x), 0.0f), fmaxf(fmaxf(lo.y, -hi.y), 0.0f), fmaxf(fmaxf(lo.z, -hi.z), 0.0f));
+                    const v3 N = fcross(ac, ab), mid = plane(4), across = plane(5), up = plane(6);
+                    const float len = s_plane[4].w, sab = sum1(ab), sac = sum1(ac);
+                    const float det = fabsf(fdot(mid, N)) - fabsf(fdot(across, N)) - fabsf(fdot(up, N)) - 1e-5f * len * sab * sac;
+                    const float off = __fdividef(2e-6f * sab * sac * (sum1(tv) + sab + sac) * len, fmaxf(det, 1e-4f * len));
+                    const float near = 0.9999f * length(gap) - off;
                     s_tri[4 * at] = make_float4(ab.x, ab.y, ab.z, ac.x);
                     s_tri[4 * at + 1] = make_float4(ac.y, ac.z, tv.x, tv.y);
                     s_tri[4 * at + 2] = make_float4(tv.z, qv.x, qv.y, qv.z);
@@ -1043,7 +1059,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                     if (listed) {
                         const Corners K = make_corners(cm, pw, ph, 4, 2, H);
                         float tMin = valid && !walk ? 1e6f : 0.0f;  // (a lane at 0 hits nothing)
-                        float second = 1e6f;  // the nearest hit but for the best one
+                        float second = 1e6f;  // no hit but the best one is nearer
                         int best = -1;
                         // moller_trumbore on a prepared triangle, in two parts.  First the numerators
                         // against the determinant, by more than rounding: a division only for
@@ -1081,11 +1097,12 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                             if (!(t > 0.0f)) return;
                             take(c, t, D);
                         };
+                        float far = 1e6f;
                         for (int side = 0; side < 2; ++side) {
                             const int c0 = !side ? 0 : own ? nf : kCand - nb, c1 = c0 + (side ? nb : nf);
                             for (int cb = c0 + 32 * part; cb < c1; cb += 32 * HALVES) {
-                                // what lies behind every ray's hit so far is left out
-                                const float far = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(tMin)));
+                                // what lies behind every ray's hit so far, and a little more, is left out
+                                far = 1.00001f * __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(tMin)));
                                 int c = cb + lane;
                                 bool in = c < c1;
                                 if (in) {
@@ -1106,6 +1123,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                                 }
                             }
                         }
+                        second = fminf(second, far);  // (the hits left out are behind this)
                         if constexpr (HALVES == 2) {
                             // the first warp takes the second's hits as it would one triangle's
                             if (part == 1) {

@@ -3,8 +3,9 @@ against the reference-shaped renderer, which traverses every ray: the same depth
 from each of its three kernels -- tiles of 16 (many pixels), tiles of 8, and tiles of 8 with
 two warps a patch (few pixels) -- for every kind of camera, where a tile has more triangles
 than its list (quarters, rays traversed one by one), behind narrow lenses, where triangles
-are hit at the same distance, without the arrays that the ray-cast can do without, and on a
-tree deeper than the traversal's stack."""
+are hit at the same distance, where leaves box another face than the one they hold, on
+triangles seen edge on, without the arrays that the ray-cast can do without, and on a tree
+deeper than the traversal's stack."""
 
 import ctypes as C
 
@@ -166,6 +167,44 @@ def test_equally_near_triangles(gpu, kernel, res):
             v.append([c, b, d])
         m, bvh = _triangles(v)
         differ, hit = _differ(m, bvh, res, 60.0, np.zeros((1, 3)), np.array([[0.0, 0.0, 0.0, 1.0]]), 2)
+        assert differ == 0 and hit > 1000, f"seed {seed}: {differ} pixels differ, {hit} are hit"
+
+
+@pytest.mark.parametrize("kernel,envs,res", [("8x2", 2, 128), ("8", 3, 160), ("16", 40, 128)])
+@pytest.mark.parametrize("foreign", [0.02, 0.5])
+def test_leaves_that_box_another_face(gpu, kernel, envs, res, foreign):
+    # refit_source: a leaf's box is another face's, nearer or farther than what it holds
+    assert _kernel(envs, res) == kernel
+    meshes = [_mesh("plain")] * envs
+    m, _ = sc.liver_model("cuda:0", envs, meshes=meshes)
+    bvh = SimBVH("cuda:0", m)
+    rng = np.random.Generator(np.random.PCG64(envs))
+    n = m.numAllVisFaces
+    src = np.arange(n, dtype=np.int32)
+    pick = rng.random(n) < foreign
+    src[pick] = rng.integers(0, n, size=int(pick.sum()))
+    bvh.refitSource = torch.as_tensor(src, device="cuda:0")
+    bvh.desc.refit_source = L.ptr(bvh.refitSource)
+    bvh.refitBVH()
+    for seed in range(4):
+        _compare(m, bvh, meshes, envs, res, "out", 4, seed)
+
+
+@pytest.mark.parametrize("kernel,res", [("8x2", 128), ("8", 256), ("16", 512)])
+@pytest.mark.parametrize("depth", [1.0, 5.0])
+def test_grazing_triangles(gpu, kernel, res, depth):
+    # triangles that run along the rays: the test's determinant goes down to its limit, and the
+    # distance it finds is off by up to some per cent, to both sides of the triangle's box
+    assert _kernel(1, res) == kernel
+    for seed in range(6):
+        rng = np.random.Generator(np.random.PCG64(seed))
+        n = 1500
+        a = np.concatenate([0.12 * rng.normal(size=(n, 2)), np.full((n, 1), -1.0)], axis=1) * rng.uniform(5.0, 40.0, (n, 1))
+        u = a / np.linalg.norm(a, axis=1, keepdims=True)
+        off = [u * rng.uniform(0.3, 1.0, (n, 1)) * depth * rng.choice([-1, 1], (n, 1)) +
+               0.5 * rng.normal(size=(n, 3)) * np.exp(rng.uniform(-4.0, 0.0, (n, 1))) for _ in range(2)]
+        m, bvh = _triangles(np.stack([a, a + off[0], a + off[1]], axis=1))
+        differ, hit = _differ(m, bvh, res, 21.73, np.zeros((1, 3)), np.array([[0.0, 0.0, 0.0, 1.0]]), 2)
         assert differ == 0 and hit > 1000, f"seed {seed}: {differ} pixels differ, {hit} are hit"
 
 
