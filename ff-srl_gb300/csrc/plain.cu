@@ -21,6 +21,8 @@ constexpr int kFourLanes = 100000;  // the most triangles k_collide takes four l
 // lets the next one start, loads what no kernel of the step writes (indices, rest values,
 // masses, flags, the instrument), and then waits -- every thread, so that a kernel cannot
 // complete before the one ahead of it has -- until the writes of the one before are seen.
+// A constraint that is switched off (a triangle that is a hole) may name no vertex or env at all:
+// what is loaded through its ids before the wait is vertex or env 0's.
 // The step's first launch starts after all earlier work, as usual.  A step of 8 x 10
 // iterations took 3,234 us on one mixed env, 4,382 on 16 and 19.8 ms on 256; with the early
 // starts 1,737, 3,296 and 17.9 ms, with the shared launches (7 an iteration became 4) 1,186,
@@ -84,6 +86,7 @@ __global__ void k_volume_xpbd(const float* xp, float* dp, int* cnt, float* lam,
     if (t < n) {
         active = active_tet[t];
         id = reinterpret_cast<const int4*>(tet)[t];
+        if (!(active == 1.0f)) id = make_int4(0, 0, 0, 0);
         rv = rest[t];
         mA = inv_mass[id.x]; mB = inv_mass[id.y]; mC = inv_mass[id.z]; mD = inv_mass[id.w];
     }
@@ -131,8 +134,9 @@ struct Edges {
 __device__ __forceinline__ void tet_constraints(const float* xp, float* dp, int* cnt, const float* __restrict__ inv_mass,
                                                 const Tets& a, bool volume, bool neo, int t) {
     const int tt = t < a.n ? t : 0;  // (n > 0: a thread past the end loads the first tet's)
-    const int4 id = __ldg(reinterpret_cast<const int4*>(a.tet) + tt);
+    int4 id = __ldg(reinterpret_cast<const int4*>(a.tet) + tt);
     const float rv = __ldg(a.rest + tt), active = volume ? __ldg(a.active + tt) : 0.0f;
+    if (!neo && !(active == 1.0f)) id = make_int4(0, 0, 0, 0);
     const float mA = __ldg(inv_mass + id.x), mB = __ldg(inv_mass + id.y), mC = __ldg(inv_mass + id.z), mD = __ldg(inv_mass + id.w);
     float d00 = 0.0f, d01 = 0.0f, d02 = 0.0f, d10 = 0.0f, d11 = 0.0f, d12 = 0.0f, d20 = 0.0f, d21 = 0.0f, d22 = 0.0f;
     if (neo) {
@@ -209,7 +213,8 @@ __device__ __forceinline__ void edge_constraint(const float* xp, float* dp, int*
                                                 const Edges& a, int e) {
     const int ee = e < a.n ? e : 0;
     const float active = __ldg(a.active + ee), L0 = __ldg(a.rest + ee);
-    const int2 id = __ldg(reinterpret_cast<const int2*>(a.edge) + ee);
+    int2 id = __ldg(reinterpret_cast<const int2*>(a.edge) + ee);
+    if (active == 0.0f) id = make_int2(0, 0);
     const float mA = __ldg(inv_mass + id.x), mB = __ldg(inv_mass + id.y);
     wait_for_previous();
     if (e >= a.n || active == 0.0f) return;
@@ -248,6 +253,7 @@ __global__ void k_distance_xpbd(const float* xp, float* dp, int* cnt, float* lam
     if (e < n) {
         active = active_edge[e];
         id = reinterpret_cast<const int2*>(edge)[e];
+        if (active == 0.0f) id = make_int2(0, 0);
         L0 = rest[e];
         mA = inv_mass[id.x]; mB = inv_mass[id.y];
     }
@@ -356,6 +362,7 @@ __global__ void k_collide(const float* xp, float* cdp, const int* __restrict__ t
     if (f < n) {
         env = t2e[f];
         open = hole[f] == 1;
+        if (open) env = 0;
         a = tri[3 * f]; b = tri[3 * f + 1]; c = tri[3 * f + 2];
     }
     auto capsule = [&](int i) { return 4ll * env + (L == 4 ? min(lane, 2) : i); };
