@@ -1457,6 +1457,8 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
     b->env_class.assign(N, -1);
     std::vector<std::vector<int>> members;
     std::vector<int> keys;  // (cluster size, mode, band)
+    struct Largest { int nv, nx; };
+    std::vector<Largest> largest;  // vertices and exchange words of a class's parts
     auto mode_for = [&](int nv) {
         if (precision == 64) return plan_smem(b, 0, nv) <= dyn_budget ? 0 : 2;
         if (plan_smem(b, 0, nv) <= dyn_budget) return 0;
@@ -1468,11 +1470,17 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
         int band = 0;
         while (part_nv[e] > bands[band]) ++band;
         int key = split[e] > 1 ? split[e] * 64 + m * 16 : m * 16 + (m == 0 ? band : 0);
-        auto it = std::find(keys.begin(), keys.end(), key);
-        int ci;
-        if (it == keys.end()) { keys.push_back(key); members.emplace_back(); ci = (int)keys.size() - 1; }
-        else ci = (int)(it - keys.begin());
+        // a class's blocks hold its largest part and its longest exchange table, which may be
+        // two envs': a split env that does not fit the class with them begins another
+        auto joins = [&](int k) {
+            return keys[k] == key && (split[e] == 1 || plan_smem(b, 0, std::max(largest[k].nv, part_nv[e])) + 8 +
+                                                               4 * (size_t)std::max(largest[k].nx, part_nx[e]) <= dyn_budget);
+        };
+        int ci = 0;
+        while (ci < (int)keys.size() && !joins(ci)) ++ci;
+        if (ci == (int)keys.size()) { keys.push_back(key); members.emplace_back(); largest.push_back({0, 0}); }
         members[ci].push_back(e);
+        largest[ci] = {std::max(largest[ci].nv, part_nv[e]), std::max(largest[ci].nx, part_nx[e])};
     }
     // the largest clusters are launched first, while they find enough SMs free side by side,
     // then the class with the costliest block: its blocks would otherwise wait for those of
@@ -1484,7 +1492,8 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
     std::iota(order.begin(), order.end(), 0);
     std::sort(order.begin(), order.end(), [&](int a, int c) {
         if (keys[a] / 64 != keys[c] / 64) return keys[a] > keys[c];
-        return block_cost[a] != block_cost[c] ? block_cost[a] > block_cost[c] : keys[a] < keys[c];
+        if (block_cost[a] != block_cost[c]) return block_cost[a] > block_cost[c];
+        return keys[a] != keys[c] ? keys[a] < keys[c] : a < c;
     });
     size_t scratch_total = 0;
     for (int oi : order) {
