@@ -261,8 +261,9 @@ int32_t refit_fused(const ffsrl_bvh& b, const float* pts, const int32_t* faces, 
     // up to an env per SM a block has the SM's shared memory (trees to 14,300 nodes) and 1,024
     // threads; with more, two blocks share it (7,100 nodes)
     const bool few = n <= sms;
-    const int smem = (few ? most : most / 2) - 1024 - 256;
-    FFSRL_CUDA_TRY(cudaFuncSetAttribute(k_refit_climb, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int limit = most - 1024 - 256, smem = few ? limit : most / 2 - 1024 - 256;
+    // (always the largest: the attribute is the function's, whichever thread set it last)
+    FFSRL_CUDA_TRY(cudaFuncSetAttribute(k_refit_climb, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
     k_refit_climb<<<n, few ? 1024 : 512, smem, s>>>(b, ids, smem);
     return FFSRL_OK;
 }
