@@ -6,6 +6,7 @@
 // bit for bit whenever the summation order is the same (the fused paths).
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 #include "ffsrl_internal.h"
 #include "vecmath.cuh"
@@ -98,11 +99,11 @@ __global__ void k_refit_level(ffsrl_bvh b, const float* __restrict__ pts, const 
     else refit_inner_global(b, b.env_node_offset[e], node, left);
 }
 
-// The fused refit runs in two launches: every leaf of every env (or listed env) at once, one
-// thread a node, then the inner nodes of an env by one block.  (One block that did an env's
-// leaves and levels in turn waited for global memory some five times a level: with cold caches
-// 72 us for one env of 2,180 faces, 101 for 8 of 1,400 to 4,400, 112 for 256; the two launches
-// take 34, 51 and 94.)
+// The fused refit of up to two envs an SM runs in two launches (see refit_fused for the others):
+// every leaf of every env (or listed env) at once, one thread a node, then the inner nodes of an
+// env by one block.  (One block that did an env's leaves and levels in turn waited for global
+// memory some five times a level: 1 and 64 envs of 1,791 nodes 27 and 31 us, of 8,919 81 and 94;
+// the two launches take 19 and 21, 50 and 61.)
 __global__ void __launch_bounds__(256) k_refit_leaves(ffsrl_bvh b, const float* __restrict__ pts,
                                                       const int* __restrict__ faces, const int* __restrict__ ids,
                                                       int chunks) {
@@ -129,8 +130,11 @@ __host__ __device__ inline size_t climb_bytes(int nn) {
 // ahead, and leaves what goes to global memory to a last pass over all pairs.  The same box
 // whichever child comes second: the left child's box is always the first operand.  An env
 // whose tree is numbered in another way or does not fit the block's shared memory is refitted
-// level by level from global memory.
-__global__ void __launch_bounds__(1024) k_refit_climb(ffsrl_bvh b, const int* __restrict__ ids, int smem_bytes) {
+// level by level from global memory.  LEAVES: the block does its env's leaves first.
+template <bool LEAVES>
+__global__ void __launch_bounds__(LEAVES ? 256 : 1024) k_refit_climb(ffsrl_bvh b, const float* __restrict__ pts,
+                                                                     const int* __restrict__ faces, const int* __restrict__ ids,
+                                                                     int smem_bytes) {
     extern __shared__ float climb_smem[];
     __shared__ int s_bad;
     const int e = ids ? ids[blockIdx.x] : blockIdx.x;
@@ -143,6 +147,11 @@ __global__ void __launch_bounds__(1024) k_refit_climb(ffsrl_bvh b, const int* __
     unsigned short* left = reinterpret_cast<unsigned short*>(arrived + nn / 64 + 1);  // kNone: a leaf
     unsigned short* parent = left + nn;
     const bool fits = nn < 65535 && (nn & 1) && climb_bytes(nn) <= (size_t)smem_bytes;
+    if (LEAVES) {
+        for (int node = threadIdx.x; node < nn; node += step)
+            if (b.left_node[n0 + node] < 0) refit_leaf(b, pts, faces, e, n0, b.topo_tri_offset[topo], base, node);
+        __syncthreads();
+    }
     if (fits) {
         if (threadIdx.x == 0) s_bad = 0;
         for (int i = threadIdx.x; i < nn; i += step) parent[i] = kNone;
@@ -249,22 +258,45 @@ __global__ void __launch_bounds__(1024) k_refit_climb(ffsrl_bvh b, const int* __
     }
 }
 
-// Both launches for n envs (ids null: all)
+// n envs (ids null: all).  What is fastest depends on their number and size (us; the climb after
+// a launch of its own for the leaves, the climb with its leaves, the levels with their leaves):
+//     nodes  envs: 1               64             216            512            1,024          2,048
+//     383    14.0 11.1 12.7   15.0 12.5 12.8   16.8 14.3 14.9   23.0 17.2 18.7   33.4 29.2 32.7   51.8 46.9 48.7
+//     1,791  18.9 27.6 23.6   21.0 30.9 27.1   31.6 35.5 32.7   57.9 52.4 45.6   112  105  105    211  177  167
+//     4,325  30.0 60.9 47.7   35.5 66.1 51.2   62.5 81.1 65.5   134  186  114    244  299  241
+//     8,919  50.3 116  84.6   60.5 123  92.8   154  181  149    320  374  248
+// With few envs a small tree is a matter of one launch or two, a larger one of the trips to global
+// memory; from two envs an SM on (at 300 of 2,557 nodes 45.7, 51.8 and 41.4, at 300 of 4,325 75, 95
+// and 80) blocks hide one another's trips, and the levels' do the least work.
 int32_t refit_fused(const ffsrl_bvh& b, const float* pts, const int32_t* faces, const int32_t* ids, int n, cudaStream_t s) {
     int dev = 0, sms = 0, most = 0;
     FFSRL_CUDA_TRY(cudaGetDevice(&dev));
     FFSRL_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     FFSRL_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const int mean = b.total_env_nodes / b.num_envs;
+    // up to an env per SM a block of the climb may have the SM's shared memory (trees to 14,300
+    // nodes) and 1,024 threads; with more, two blocks share it (7,100 nodes)
+    const bool few = n <= sms;
+    const int limit = most - 1024 - 256, share = few ? limit : most / 2 - 1024 - 256;
+    if (n > 2 * sms || (!few && climb_bytes(mean) > (size_t)share)) {
+        k_refit_climb<true><<<n, 256, 0, s>>>(b, pts, faces, ids, 0);
+        return FFSRL_OK;
+    }
+    // no tree has more nodes than all topologies together, but one of each other
+    const int others = std::max(b.num_topologies, 1) - 1;
+    const int largest = b.total_topology_nodes > others ? b.total_topology_nodes - others : INT_MAX;
+    if (largest <= 512) {
+        const int smem = (int)climb_bytes(largest);  // (8 KB: no limit to raise)
+        k_refit_climb<true><<<n, 256, smem, s>>>(b, pts, faces, ids, smem);
+        return FFSRL_OK;
+    }
     const int chunks = std::max(1, std::min(mean / 256 + 1, 64));
     k_refit_leaves<<<(unsigned)((long long)chunks * n), 256, 0, s>>>(b, pts, faces, ids, chunks);
-    // up to an env per SM a block has the SM's shared memory (trees to 14,300 nodes) and 1,024
-    // threads; with more, two blocks share it (7,100 nodes)
-    const bool few = n <= sms;
-    const int limit = most - 1024 - 256, smem = few ? limit : most / 2 - 1024 - 256;
+    const int smem = (int)std::min((size_t)share, climb_bytes(largest));
     // (always the largest: the attribute is the function's, whichever thread set it last)
-    FFSRL_CUDA_TRY(cudaFuncSetAttribute(k_refit_climb, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
-    k_refit_climb<<<n, few ? 1024 : 512, smem, s>>>(b, ids, smem);
+    FFSRL_CUDA_TRY(cudaFuncSetAttribute(k_refit_climb<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    const int threads = std::min(few ? 1024 : 512, std::max(128, (largest / 2 + 31) / 32 * 32));  // a pair each
+    k_refit_climb<false><<<n, threads, smem, s>>>(b, pts, faces, ids, smem);
     return FFSRL_OK;
 }
 
