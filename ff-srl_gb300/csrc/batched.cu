@@ -1712,6 +1712,13 @@ extern "C" int32_t ffsrl_batch_class_envs(const ffsrl_batch* b, int32_t cls, int
     return FFSRL_OK;
 }
 
+extern "C" int32_t ffsrl_batch_class_split(const ffsrl_batch* b, int32_t cls, int32_t* blocks_per_env) {
+    if (!b || !blocks_per_env || cls < 0 || cls >= (int)b->classes.size())
+        return fail(FFSRL_ERR_INVALID_ARGUMENT, "ffsrl_batch_class_split");
+    *blocks_per_env = b->classes[cls].split;
+    return FFSRL_OK;
+}
+
 extern "C" int32_t ffsrl_batch_set_class_prefetch(ffsrl_batch* b, int32_t cls, int32_t kind) {
     if (!b || cls < 0 || cls >= (int)b->classes.size() || kind < 0 || kind > 2)
         return fail(FFSRL_ERR_INVALID_ARGUMENT, "ffsrl_batch_set_class_prefetch");

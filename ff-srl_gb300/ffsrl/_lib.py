@@ -182,6 +182,7 @@ def lib() -> C.CDLL:
         "ffsrl_batch_state_f64": ([P, P], I32),
         "ffsrl_batch_class_info": ([P, I32, C.POINTER(I32), C.POINTER(I32), C.POINTER(I32), C.POINTER(I32)], I32),
         "ffsrl_batch_class_envs": ([P, I32, P], I32),
+        "ffsrl_batch_class_split": ([P, I32, P], I32),
         "ffsrl_batch_set_class_block": ([P, I32, I32], I32),
         "ffsrl_batch_set_class_prefetch": ([P, I32, I32], I32),
         "ffsrl_create": ([pm, pp, I32, C.POINTER(P)], I32),

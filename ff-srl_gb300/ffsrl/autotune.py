@@ -5,7 +5,9 @@ For each class this times the class's environments for one step at every block s
 that has a kernel instantiation and fits on an SM, with and without the L1 prefetch of
 the tet records, keeps the fastest, and records the
 choice in a JSON cache keyed by the device and the class's shape, so later plans with
-the same classes skip the timing.  The model's state is saved before and restored after
+the same classes skip the timing.  Whether a class's environments are divided among a
+cluster of blocks hangs on the whole plan, so that is part of the key; a divided class's
+kernels have fewer block sizes and one way to fetch the records.  The model's state is saved before and restored after
 the timing runs.
 """
 
@@ -24,6 +26,7 @@ from ._lib import FFSRLError, check, lib
 
 CANDIDATES = (128, 256, 512, 640, 768, 1024)
 PREFETCH = (0, 1, 2)  # next tet record: not fetched ahead, into L1, into registers
+DIVIDED_CANDIDATES, DIVIDED_PREFETCH = (128, 256, 512, 768), (0,)
 
 
 def cache_path() -> Path:
@@ -37,9 +40,12 @@ def _classes(plan):
     for c in range(n):
         mx, mode, blk, ne = C.c_int32(), C.c_int32(), C.c_int32(), C.c_int32()
         check(lib().ffsrl_batch_class_info(plan.handle, c, C.byref(mx), C.byref(mode), C.byref(blk), C.byref(ne)))
+        split = C.c_int32()
+        check(lib().ffsrl_batch_class_split(plan.handle, c, C.byref(split)))
         ids = np.zeros(max(ne.value, 1), dtype=np.int32)
         check(lib().ffsrl_batch_class_envs(plan.handle, c, ids.ctypes.data))
-        out.append({"max_nv": mx.value, "mode": mode.value, "block": blk.value, "envs": ids[:ne.value]})
+        out.append({"max_nv": mx.value, "mode": mode.value, "block": blk.value, "split": split.value,
+                    "envs": ids[:ne.value]})
     return out
 
 
@@ -47,8 +53,8 @@ def _key(plan, cls) -> str:
     m = plan.model
     props = torch.cuda.get_device_properties(m.device)
     tets = int(sum(int(m.envTetStart[e + 1] - m.envTetStart[e]) for e in cls["envs"]))
-    sig = f"v5|{props.name}|{props.multi_processor_count}|{m.constraintFlags}|{m.simSubsteps}|{m.simConstraints}|" \
-          f"{cls['mode']}|{cls['max_nv']}|{len(cls['envs'])}|{tets}|{plan.precision}|" \
+    sig = f"v6|{props.name}|{props.multi_processor_count}|{m.constraintFlags}|{m.simSubsteps}|{m.simConstraints}|" \
+          f"{cls['mode']}|{cls['max_nv']}|{cls['split']}|{len(cls['envs'])}|{tets}|{plan.precision}|" \
           f"{getattr(plan, 'arithmetic', '')}|{getattr(plan, 'accumulation', '')}"
     return hashlib.sha1(sig.encode()).hexdigest()[:16]
 
@@ -89,11 +95,12 @@ def autotune(plan, reps: int = 2, use_cache: bool = True, verbose: bool = False)
                                "cached": True})
                 continue
             best = None
-            for b in CANDIDATES:
+            divided = cls["split"] > 1
+            for b in DIVIDED_CANDIDATES if divided else CANDIDATES:
                 check(lib().ffsrl_batch_set_class_prefetch(plan.handle, ci, 0))
                 if lib().ffsrl_batch_set_class_block(plan.handle, ci, b) != 0:
                     continue
-                for pf in PREFETCH:
+                for pf in DIVIDED_PREFETCH if divided else PREFETCH:
                     if lib().ffsrl_batch_set_class_prefetch(plan.handle, ci, pf) != 0:
                         continue
                     ms = _time(plan, cls["envs"], reps)

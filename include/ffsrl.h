@@ -388,6 +388,9 @@ int32_t ffsrl_batch_info(const ffsrl_batch* b, int64_t* device_bytes, int32_t* n
 int32_t ffsrl_batch_class_info(const ffsrl_batch* b, int32_t cls, int32_t* max_nv, int32_t* mode, int32_t* block,
                                int32_t* num_envs);
 int32_t ffsrl_batch_class_envs(const ffsrl_batch* b, int32_t cls, int32_t* env_ids);
+/* How many blocks step one env of class cls: 1, or the size of the cluster its envs are divided
+   among. */
+int32_t ffsrl_batch_class_split(const ffsrl_batch* b, int32_t cls, int32_t* blocks_per_env);
 int32_t ffsrl_batch_set_class_block(ffsrl_batch* b, int32_t cls, int32_t block);
 /* Autotuner hook, how class cls's kernel fetches each thread's next tet record one loop
    trip ahead: 0 not at all, 1 into L1 (prefetch.global.L1), 2 into registers (block sizes
