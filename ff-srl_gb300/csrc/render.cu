@@ -867,7 +867,7 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 // test computes from the camera and the triangle alone, the faces towards the camera first);
 // then each warp takes patches of 4 x 2 pixels (32 rays), keeps the listed triangles its
 // patch's rays can reach, a triangle a lane, and tests them one after another, all lanes the
-// same triangle.  A tile with more triangles than the list holds is done in quarters.
+// same triangle.  A tile of 16 with more triangles than the list holds is done in quarters.
 // 256 envs of 500-20,000 tets at 128 x 128: a thread per ray took 1,224 us and 1,900
 // instructions a warp of 32 rays with two thirds of its lanes busy, the tiles 730; 8 textured
 // envs at 512 x 512: 540 and 275 us.  What bounds it now is issue, 65% of it, and on one env
@@ -881,15 +881,17 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 // test at the end.  In the rare case that the test fails, or puts the entry no nearer than another
 // hit (two triangles hit in a box's corner, or at the same distance in a plane that bounds their
 // boxes, where the one that is kept hangs on the order of the traversal), the ray is traversed.
-// So is a ray along a coordinate plane, and every ray of a 4 x 4 tile that still has too many
-// triangles, or of a tree deeper than kSteps levels below the ones tested first.
+// So is a ray along a coordinate plane, and every ray of an 8 x 8 tile that has too many triangles
+// (quarters of those took up to 1.7 times as long), or of a tree deeper than kSteps levels below
+// the ones tested first.
 constexpr int kCand = 448;      // triangles of a tile, 64 bytes of shared memory each
 constexpr int kFront = 768;     // nodes of a level
 constexpr int kSteps = 40;
 constexpr int kTwoWarps = 608;  // the most tiles of 8 whose patches take two warps each
 constexpr int kList = 160;      // triangles a warp keeps for its four patches
-// Levels tested at once at the start.  Large images (T 16): at most 255 nodes, one a thread.
-// Small ones wait for each step more than for its work: at most 2,047 nodes, eight a thread.
+// Levels tested at once at the start.  Tiles of 16, which fill the GPU: at most 255 nodes, one a
+// thread.  Tiles of 8, taken for less work, wait for each step more than for what it does: at most
+// 2,047 nodes, eight a thread.
 template <int T> struct FirstLevel { static constexpr int value = T == 16 ? 7 : 10; };
 
 // The traversal of one ray, kept out of line: few rays take it
@@ -912,7 +914,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
     // the tile's planes; its middle ray and the longest ray's length, half its width and height
     __shared__ float4 s_plane[7];
     __shared__ int s_n[3], s_leaves, s_over, s_nf, s_nb;
-    __shared__ int s_todo[8][3];  // tiles still to do: x, y, size
+    __shared__ int s_todo[4][2];  // quarters still to do: x, y
     __shared__ float s_hit[HALVES == 2 ? 8 : 1][3][HALVES == 2 ? 32 : 1];  // the second warp's rays: distance, second, triangle
     constexpr int kThreads = 256 * HALVES;
     const int R = r.resolution, W = 2 * R, H = 2 * R;
@@ -955,6 +957,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
             for (int i = 0; i < 4; ++i) F.n[i] = plane(i);
             auto visit = [&](int node, int* count, int* front, bool expand) {
                 if ((unsigned)node >= (unsigned)ev.nn) { s_over = 1; return; }
+                if (*(volatile int*)&s_over) return;  // (the lists are given up: nothing more to find)
                 const float4 a = __ldg(ev.box + 2 * node), c = __ldg(ev.box + 2 * node + 1);
                 const int left = __float_as_int(a.w);
                 if (left != -1 && !expand) return;
@@ -962,6 +965,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                 if (left == -1) {
                     const int q = atomicAdd(&s_leaves, 1);
                     if (q < kCand) s_leaf[q] = node;
+                    else s_over = 1;
                 } else {
                     const int q = atomicAdd(count, 2);
                     if (left >= 0 && left + 1 < ev.nn && q + 1 < kFront) {
@@ -1000,7 +1004,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                 __syncthreads();
             }
             if (step == kSteps && tid == 0) s_over = 1;
-            const int leaves = min(s_leaves, kCand);
+            const int leaves = s_over ? 0 : s_leaves;
             for (int i = tid; i < leaves; i += kThreads) {
                 const int node = s_leaf[i];
                 const int fc = __float_as_int(__ldg(ev.box + 2 * node + 1).w), first = fc >> 8;
@@ -1034,16 +1038,15 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
         }
         __syncthreads();
         int nf = s_nf, nb = s_nb;  // triangles facing the camera, and others
-        const bool listed = packed && !s_over && s_leaves <= kCand && nf + nb <= kCand;
-        if (packed && !listed && size > 4) {
-            // the quarters instead (at most 3 + 4 tiles wait at a time)
-            size >>= 1;
+        const bool listed = packed && !s_over && nf + nb <= kCand;
+        if (packed && !listed && size > 8) {
+            // the quarters instead
+            size = 8;
             if (tid < 4) {
-                s_todo[todo + tid][0] = tx + (tid & 1) * size;
-                s_todo[todo + tid][1] = ty + (tid >> 1) * size;
-                s_todo[todo + tid][2] = size;
+                s_todo[tid][0] = tx + (tid & 1) * 8;
+                s_todo[tid][1] = ty + (tid >> 1) * 8;
             }
-            todo += 4;
+            todo = 4;
         } else {
             // the triangles of the list from which a warp's rays can hit, by lane: whether triangle
             // c is one of them for the rays between corners k
@@ -1054,8 +1057,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
             // a warp's patches: four of 4 x 2 pixels in a region of 8 x 4 (tiles of 16), or one.
             // The region's triangles are picked from the tile's first, a patch's from those.
             const bool four = T == 16 && size == 16;
-            const int rx = tx + (size == 4 ? 0 : (warp & 1) * (four ? 8 : 4));
-            const int ry = ty + (size == 4 ? warp * 2 : (warp >> 1) * (four ? 4 : 2));
+            const int rx = tx + (warp & 1) * (four ? 8 : 4), ry = ty + (warp >> 1) * (four ? 4 : 2);
             bool own = false;  // the warp's list is s_list, or the tile's
             if (four && listed && nf + nb > 32) {
                 const Corners K = make_corners(cm, rx, ry, 8, 4, H);
@@ -1074,7 +1076,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                 if (n <= kList) { own = true; nf = f; nb = n - f; }
                 __syncwarp();
             }
-            for (int patch = 0; patch < (four ? 4 : 1) && (size > 4 || warp < 2); ++patch) {
+            for (int patch = 0; patch < (four ? 4 : 1); ++patch) {
                 const int pw = rx + (patch & 1) * 4, ph = ry + (patch >> 1) * 2;
                 const int j = lane >> 2, q = lane & 3;
                 const int px = pw + (j & 3), py = ph + (j >> 2);
@@ -1197,7 +1199,7 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
         if (todo == 0) return;
         __syncthreads();
         --todo;
-        tx = s_todo[todo][0]; ty = s_todo[todo][1]; size = s_todo[todo][2];
+        tx = s_todo[todo][0]; ty = s_todo[todo][1];
     }
 }
 
