@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdint>
 #include "ffsrl_internal.h"
 #include "vecmath.cuh"
@@ -887,7 +888,6 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 constexpr int kCand = 448;      // triangles of a tile, 64 bytes of shared memory each
 constexpr int kFront = 768;     // nodes of a level
 constexpr int kSteps = 40;
-constexpr int kTwoWarps = 608;  // the most tiles of 8 whose patches take two warps each
 constexpr int kList = 160;      // triangles a warp keeps for its four patches
 // Levels tested at once at the start.  Tiles of 16, which fill the GPU: at most 255 nodes, one a
 // thread.  Tiles of 8, taken for less work, wait for each step more than for what it does: at most
@@ -1226,24 +1226,45 @@ __global__ void __launch_bounds__(256) k_rays_alone(const __grid_constant__ ffsr
     store_pixel(r, s, valid, e, px, py);
 }
 
-// Tiles of 16 pixels share the walk among 32 patches; tiles of 8, four times as many, where
-// those of 16 would give an SM fewer than seven.  Where even those are few, the time is that of
-// the patch with the most triangles, some 70,000 cycles of tests on one warp: two warps share
-// its triangles (one env at 128 x 128, 256 tiles, 56 -> 46 us; two 56 -> 48; with four, 1,024
-// tiles, there is 3% in it, with fifteen it costs 10%).
-// In small images a tile holds much of the mesh and its rays share little: each ray is
-// traversed alone (16 x 16, 1 and 216 envs: 43 and 91 us, by tiles 75 and 180; 50 x 50, 24 and
-// 216: 75 and 235, by tiles 127 and 331; 64 x 64, 24 and 216: 81 and 317, by tiles 139 and 349).  So
-// are images of up to 128 pixels where the tiles are too few to hide one another's chains (24
-// envs of 500-15,000 tets, 80, 100 and 128 pixels: 96, 120 and 154 us, by tiles 162, 177 and 174;
-// 216 envs at 128: 1,007 and 710; one env at 128: 70 and 43).
+// Which kernel is fastest hangs on how densely a tile's pixels are covered with triangles and on
+// how much there is to do.  What the sizes tell of both: `dense`, an env's nodes (about its
+// triangles) over the pixels of a unit angle's square, and `work`, those pixels over all envs.
+// Time over that of a thread per ray, mean and worst, of 8 x 8 tiles with two warps a patch, of
+// 8 x 8 and of 16 x 16 tiles (1,116 images of ellipsoids of 500-46,640 tets with their instrument,
+// alone and mixed, 1 to 216 envs, 72 to 700 pixels, lenses of 22, 40 and 60 degrees):
+//     dense  work < 100,000              to 200,000                  to 800,000                  to 2.4 million              above
+//     < .02                              0.56 0.6  0.57 0.6  1.1 1.3 0.68 1.2  0.60 0.8  1.0 1.4 0.84 1.5  0.64 1.0  0.7 1.1 1.1 1.6  0.68 1.1  0.47 0.9
+//     < .08  0.66 0.8  0.76 1.0  1.5 1.8 0.67 1.1  0.75 1.2  1.4 2.6 0.70 1.1  0.68 1.1  1.2 1.7 0.87 1.4  0.70 1.2  0.9 1.5 1.0 1.5  0.67 1.0  0.56 1.1
+//     < .16  0.73 1.1  0.86 1.2  1.7 2.3 0.79 1.2  0.87 1.2  1.5 1.9 0.92 1.2  0.86 1.2  1.3 2.0 1.10 1.4  0.85 1.1  1.0 1.4 1.2 1.6  0.79 1.1  0.67 1.0
+//     < .32  0.83 1.1  0.93 1.2  1.9 2.5 1.03 1.2  1.04 1.2  1.6 1.9 1.20 1.4  1.06 1.2  1.5 1.9 1.32 1.5  0.98 1.1  1.1 1.2 1.3 1.6  0.87 1.1  0.77 1.1
+//     more   1.03 1.2  1.09 1.2  2.1 2.4 1.18 1.3  1.18 1.2  2.0 2.5 1.34 1.5  1.14 1.2  1.7 2.4 1.48 1.7  1.09 1.2  1.3 1.6 1.5 1.7  1.00 1.2  0.99 1.3
+// Tiles of 16 want some 600 blocks, too.  Through wider lenses (100 degrees, 372 images) most
+// tiles are empty, which costs a thread per ray next to nothing: two warps a patch gain below a work
+// of 100,000 and a density of .08 (0.70, worst 0.7), tiles of 16 above 800,000 and below .16 (0.79,
+// 1.0), tiles of 8 nowhere to speak of.  In images of up to 64 pixels a tile holds much of the mesh.
+// By this rule the images of the three lenses take 0.62 of a thread per ray's time (the best kernel
+// for each 0.61), those of 100 degrees 0.97; the worst image 1.23.
 void launch_rays(const ffsrl_render& r, const ffsrl_bvh& b, const int32_t* ids, int n, cudaStream_t s) {
     auto tiles = [&](int t) { return ((long long)(r.resolution + t - 1) / t) * ((r.resolution + t - 1) / t) * n; };
-    if (r.resolution <= 64 || (r.resolution <= 128 && tiles(8) > kTwoWarps && tiles(16) < 1600))
-        k_rays_alone<<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
-    else if (tiles(16) >= 1024) k_rays<16, 1><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n);
-    else if (tiles(8) <= kTwoWarps) k_rays<8, 2><<<(unsigned)tiles(8), 512, 0, s>>>(r, b, ids, n);
-    else k_rays<8, 1><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
+    const float lens = std::max(std::fabs(r.camera_tan), std::fabs(r.camera_tan * r.camera_aspect));
+    const float per_angle = (float)r.resolution / lens, work = (float)n * per_angle * per_angle;
+    const float dense = (float)b.total_env_nodes / (float)b.num_envs / (per_angle * per_angle);
+    const bool wide = lens > 0.75f;
+    bool t16, t8x2, t8;
+    if (work >= 2.4e6f) t16 = dense < 0.64f && tiles(16) >= 600;
+    else if (work >= 1.2e6f) t16 = dense < 0.32f && tiles(16) >= 1024;
+    else t16 = wide && (work >= 8e5f ? dense < 0.16f : work >= 4e5f && dense < 0.02f);
+    if (wide) {
+        t8x2 = work < 1e5f && dense < 0.08f;
+        t8 = false;
+    } else {
+        t8x2 = (work < 2e5f && dense < 0.16f) || (work < 1e5f && dense < 0.32f);
+        t8 = dense < 0.16f;
+    }
+    if (r.resolution > 64 && t16) k_rays<16, 1><<<(unsigned)tiles(16), 256, 0, s>>>(r, b, ids, n);
+    else if (r.resolution > 64 && t8x2) k_rays<8, 2><<<(unsigned)tiles(8), 512, 0, s>>>(r, b, ids, n);
+    else if (r.resolution > 64 && t8) k_rays<8, 1><<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
+    else k_rays_alone<<<(unsigned)tiles(8), 256, 0, s>>>(r, b, ids, n);
 }
 
 int32_t check_bvh(const ffsrl_bvh* b) {
