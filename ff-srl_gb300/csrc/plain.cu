@@ -385,12 +385,12 @@ __global__ void k_collide(const float* xp, float* cdp, const int* __restrict__ t
         pA = ldw3(xp, a); pB = ldw3(xp, b); pC = ldw3(xp, c);
         // A response needs a point of the capsule's segment within its radius of a point of the
         // triangle, so there is none where the boxes are apart (the margin, 1e-4 of the
-        // coordinates, is far above their rounding).  A triangle without one adds nothing.  NaN
-        // coordinates are not apart from anything.
+        // coordinates, is far above their rounding).  A triangle without one adds nothing.  NaN and
+        // infinite coordinates are not apart from anything: their responses are NaN.
         const v3 lo = vmin(pA, vmin(pB, pC)), hi = vmax(pA, vmax(pB, pC));
         const float sum = ((pA.x + pA.y) + (pA.z + pB.x)) + ((pB.y + pB.z) + (pC.x + pC.y)) + pC.z;
         for (int i = 0; i < N; ++i)
-            if (isnan(sum) || !(lo.x > chi[i].x || lo.y > chi[i].y || lo.z > chi[i].z || hi.x < clo[i].x || hi.y < clo[i].y || hi.z < clo[i].z))
+            if (!isfinite(sum) || !(lo.x > chi[i].x || lo.y > chi[i].y || lo.z > chi[i].z || hi.x < clo[i].x || hi.y < clo[i].y || hi.z < clo[i].z))
                 near |= 1u << i;
         if (L == 4 && lane == 3) near = 0;
     }
