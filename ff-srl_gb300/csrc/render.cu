@@ -883,8 +883,8 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 // hit (two triangles hit in a box's corner, or at the same distance in a plane that bounds their
 // boxes, where the one that is kept hangs on the order of the traversal), the ray is traversed.
 // So is a ray along a coordinate plane, and every ray of an 8 x 8 tile that has too many triangles
-// (quarters of those took up to 1.7 times as long), or of a tree deeper than kSteps levels below
-// the ones tested first.
+// (quarters of those took up to 1.7 times as long) or one of extreme size, or of a tree deeper than
+// kSteps levels below the ones tested first.
 constexpr int kCand = 448;      // triangles of a tile, 64 bytes of shared memory each
 constexpr int kFront = 768;     // nodes of a level
 constexpr int kSteps = 40;
@@ -1025,9 +1025,12 @@ __global__ void __launch_bounds__(256 * HALVES, 4 / HALVES) k_rays(const __grid_
                     const v3 lo = vmin(vmin(ab, ac), mk(0.0f, 0.0f, 0.0f)) - tv, hi = vmax(vmax(ab, ac), mk(0.0f, 0.0f, 0.0f)) - tv;
                     const v3 gap = mk(fmaxf(fmaxf(lo.x, -hi.x), 0.0f), fmaxf(fmaxf(lo.y, -hi.y), 0.0f), fmaxf(fmaxf(lo.z, -hi.z), 0.0f));
                     const v3 N = fcross(ac, ab), mid = plane(4), across = plane(5), up = plane(6);
-                    const float len = s_plane[4].w, sab = sum1(ab), sac = sum1(ac);
+                    const float len = s_plane[4].w, sab = sum1(ab), sac = sum1(ac), stv = sum1(tv);
+                    // Beyond these sizes the tests below could overflow, or take for below zero what
+                    // the triangle test rounds to -0 (and NaN is left to it)
+                    if (!(sab * sac < 1e14f && stv * (sab + sac) < 1e30f)) s_over = 1;
                     const float det = fabsf(fdot(mid, N)) - fabsf(fdot(across, N)) - fabsf(fdot(up, N)) - 1e-5f * len * sab * sac;
-                    const float off = __fdividef(2e-6f * sab * sac * (sum1(tv) + sab + sac) * len, fmaxf(det, 1e-4f * len));
+                    const float off = __fdividef(2e-6f * sab * sac * (stv + sab + sac) * len, fmaxf(det, 1e-4f * len));
                     const float near = 0.9999f * length(gap) - off;
                     s_tri[4 * at] = make_float4(ab.x, ab.y, ab.z, ac.x);
                     s_tri[4 * at + 1] = make_float4(ac.y, ac.z, tv.x, tv.y);

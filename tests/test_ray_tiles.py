@@ -4,7 +4,7 @@ from each of its three kernels -- tiles of 16 (many pixels), tiles of 8, and til
 two warps a patch (few pixels) -- for every kind of camera, where a tile has more triangles
 than its list (quarters, rays traversed one by one), behind narrow lenses, where triangles
 are hit at the same distance, where leaves box another face than the one they hold, on
-triangles seen edge on, without the arrays that the ray-cast can do without, and on a tree
+triangles seen edge on, with vertices that are no numbers or overflow in products, without the arrays that the ray-cast can do without, and on a tree
 deeper than the traversal's stack."""
 
 import ctypes as C
@@ -219,6 +219,28 @@ def test_grazing_triangles(gpu, kernel, res, depth):
         assert _kernel(bvh, 1, res) == kernel
         differ, hit = _differ(m, bvh, res, 21.73, np.zeros((1, 3)), np.array([[0.0, 0.0, 0.0, 1.0]]), 2)
         assert differ == 0 and hit > 1000, f"seed {seed}: {differ} pixels differ, {hit} are hit"
+
+
+@pytest.mark.parametrize("kernel,envs,res", [("8x2", 1, 100), ("8", 2, 205), ("16", 30, 128)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf"), 1e15, -1e20, 1e25, 1e30, -1e35, -3e38])
+def test_extreme_vertices(gpu, kernel, envs, res, value):
+    mesh = mg.ellipsoid_for_tets(1500)
+    for count in (1, 5, 200):
+        m, _ = sc.liver_model("cuda:0", envs, meshes=[mesh] * envs)
+        bvh = SimBVH("cuda:0", m)
+        assert _kernel(bvh, envs, res, 60.0) == kernel
+        rng = np.random.Generator(np.random.PCG64(count))
+        m.allVisPoint.view(-1)[torch.as_tensor(rng.integers(0, m.allVisPoint.numel(), count), device="cuda:0")] = value
+        bvh.refitBVH()
+        images = []
+        for fused in (False, True):
+            r = WarpRaycastRendererDO("cuda:0", m, resolution=res, mode="headless", fused=fused, render_mode=4,
+                                      verticalAperture=sc.fov_aperture(60.0), horizontalAperture=sc.fov_aperture(60.0))
+            r.setCameras(*sc.env_cameras([mesh] * envs, seed=1))
+            r.renderNew(bvh, m)
+            torch.cuda.synchronize()
+            images.append(r.depthImages().cpu().numpy().view(np.int32))
+        assert np.array_equal(*images), f"{count}: {(images[0] != images[1]).sum()} depths differ"
 
 
 @pytest.mark.parametrize("kernel,envs,res", [("8x2", 1, 80), ("8", 2, 100), ("16", 2, 400)])
