@@ -470,8 +470,10 @@ def main():
                    "sample": f"32 envs of the same pool, 1 full env-step (8x10 solve, refit, {RES}x{RES} ray-cast), "
                              "oracle restatement, OpenMP over envs"}
         # per step: instrument kinematics, one launch per size class, remap, instrument visual points,
-        # fused refit (leaves, then the climb), normal gather, rays; per episode reset: instrument visual points, remap and grasp
-        launches = K * (n_cls + 7) + 3 * resets_timed
+        # fused refit (one launch for more than two envs an SM, else two), normal gather, rays; per episode
+        # reset: instrument visual points, remap and grasp
+        refit = 1 if envs > 2 * torch.cuda.get_device_properties(device).multi_processor_count else 2
+        launches = K * (n_cls + 5 + refit) + 3 * resets_timed
         line = {"metric": METRIC, "value": value, "unit": "env-steps/s", "n_gpus": world, "steps": K,
                 "warmup": W, "ms_per_step": total_ms / K, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded meshes and random-walk actions)",

@@ -869,9 +869,9 @@ __device__ __forceinline__ bool outside(const Bundle& b, v3 lo, v3 hi) {
 // then each warp takes patches of 4 x 2 pixels (32 rays), keeps the listed triangles its
 // patch's rays can reach, a triangle a lane, and tests them one after another, all lanes the
 // same triangle.  A tile of 16 with more triangles than the list holds is done in quarters.
-// 256 envs of 500-20,000 tets at 128 x 128: a thread per ray took 1,224 us and 1,900
-// instructions a warp of 32 rays with two thirds of its lanes busy, the tiles 730; 8 textured
-// envs at 512 x 512: 540 and 275 us.  What bounds it now is issue, 65% of it, and on one env
+// 256 envs of 500-20,000 tets at 128 x 128: a thread per ray takes 1,186 us and 1,900
+// instructions a warp of 32 rays with two thirds of its lanes busy, the tiles 747; 8 textured
+// envs at 512 x 512: 526 and 290 us.  What bounds it now is issue, 65% of it, and on one env
 // the chain of loads, tests and shading of the patch with the most triangles (45 us with one
 // warp a patch, 35 with two: launch_rays).
 //

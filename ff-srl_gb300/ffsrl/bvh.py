@@ -6,8 +6,8 @@ topology bit for bit).  The reference stores one topology for all environments a
 AABB set per environment (``bvh.py:190-196, 506-514``); here each distinct mesh gets its
 own topology, shared by every environment that uses it, so environments may differ.
 
-``refitBVH`` updates the boxes from the current visual points: by default with one
-launch (a block per environment walking its tree bottom-up); ``fused=False`` runs the
+``refitBVH`` updates the boxes from the current visual points: by default with one or two
+launches (the leaves, then a block per environment for its inner nodes); ``fused=False`` runs the
 reference's one launch per tree level (``refitBVHLoop``, ``bvh.py:419-440``).
 """
 

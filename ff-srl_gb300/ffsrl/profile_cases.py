@@ -12,7 +12,7 @@ the device, so a capture of one to six launches ends within a minute or two.
                                        # 152 copies of one 16k-tet mesh, one step with the named
                                        # constraints (e.g. VOLUME+DISTANCE; default: all)
     python -m ffsrl.profile_cases render [envs]       # refit + vertex normals + ray-cast at 128x128
-    python -m ffsrl.profile_cases plain [envs]        # one reference-shaped step (one launch per kernel)
+    python -m ffsrl.profile_cases plain [envs]        # one reference-shaped step
 
 The mixed cases draw per-env meshes from the same seeded generator as the 4096-env
 throughput workload (tet counts log-uniform in [500, 20000]), so per-env-step figures

@@ -316,7 +316,8 @@ int32_t ffsrl_bvh_build_host(const float* points, const int32_t* faces, int32_t 
                              int32_t* num_nodes, int32_t* max_level);
 /* refitBVHLoop (bvh.py:419-440): one launch of refitBVHLevel per level, deepest first. */
 int32_t ffsrl_bvh_refit_levels(const ffsrl_bvh* bvh, const float* vis_point, const int32_t* vis_face, void* stream);
-/* Same result in one launch: one block per env walks its tree bottom-up. */
+/* Same result in one or two launches, by the number of envs and the size of their trees: the
+   leaves' boxes, then each env's inner nodes by one block. */
 int32_t ffsrl_bvh_refit_fused(const ffsrl_bvh* bvh, const float* vis_point, const int32_t* vis_face, void* stream);
 
 /* ffsrl_bvh_refit_fused for the listed envs only (device array of env ids). */
@@ -327,8 +328,9 @@ int32_t ffsrl_bvh_refit_fused_envs(const ffsrl_bvh* bvh, const float* vis_point,
 /* renderFunctionNew (render.py:975-1022): zero, vertex_normal_sum (atomics), normalize,
    drawSimBVHKernelManyEnvs over (2R)^2 rays per env, downsample_kernel. */
 int32_t ffsrl_render_reference(const ffsrl_render* r, const ffsrl_bvh* bvh, void* stream);
-/* Same images: normals by CSR gather in face order, one thread per ray with a register
-   stack, the 2x2 downsample fused through warp shuffles. */
+/* Same images: normals by CSR gather in face order; the rays by tiles of pixels that share the
+   walk down the tree, or one thread per ray where tiles share little (by resolution, lens and
+   number of envs); the 2x2 downsample fused through warp shuffles. */
 int32_t ffsrl_render_fused(const ffsrl_render* r, const ffsrl_bvh* bvh, void* stream);
 
 /* ffsrl_render_fused for the listed envs only (device array of env ids): their vertex
