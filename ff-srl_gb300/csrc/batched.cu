@@ -86,6 +86,7 @@ struct ffsrl_batch {
         int split = 1;     // blocks that step one env (a cluster); max_nv is then a part's
         int env_nv = 0;    // largest env vertex count
         int prefetch = 0;  // L1 prefetch of the next tet record (autotuned)
+        bool own_block = true;  // the block size is the plan's choice, not the caller's
         int tri_cap = 0;   // surface triangles kept in shared memory per env (0: read from L2)
         size_t smem, scratch_stride, scratch_offset;
         int work_offset, work_count;
@@ -1539,6 +1540,7 @@ extern "C" int32_t ffsrl_batch_create(const ffsrl_model* hm, const ffsrl_model* 
                 }
             if (block_override <= 0) want = split_block(items);
         }
+        c.own_block = block_override <= 0;
         if (int32_t st = configure_class(b, c, want, dyn_budget)) { free_batch(b); return st; }
         // scratch for the largest grid any block size can give (8 resident blocks per SM)
         c.scratch_offset = scratch_total;
@@ -1727,7 +1729,9 @@ extern "C" int32_t ffsrl_batch_set_class_prefetch(ffsrl_batch* b, int32_t cls, i
     FFSRL_CUDA_TRY(cudaDeviceSynchronize());
     ffsrl_batch::Class c = b->classes[cls];
     c.prefetch = kind;
-    if (int32_t st = configure_class(b, c, c.block, b->dyn_budget)) return st;
+    // the plan's own 768 threads give way to 512, which have the registers for kind 2
+    const bool gives_way = kind == 2 && c.split == 1 && c.mode == 0 && c.own_block && c.block == 768;
+    if (int32_t st = configure_class(b, c, gives_way ? 512 : c.block, b->dyn_budget)) return st;
     b->classes[cls] = c;
     return FFSRL_OK;
 }
@@ -1736,6 +1740,7 @@ extern "C" int32_t ffsrl_batch_set_class_block(ffsrl_batch* b, int32_t cls, int3
     if (!b || cls < 0 || cls >= (int)b->classes.size()) return fail(FFSRL_ERR_INVALID_ARGUMENT, "ffsrl_batch_set_class_block");
     FFSRL_CUDA_TRY(cudaDeviceSynchronize());
     ffsrl_batch::Class c = b->classes[cls];
+    c.own_block = false;
     if (int32_t st = configure_class(b, c, block, b->dyn_budget)) return st;
     b->classes[cls] = c;
     return FFSRL_OK;

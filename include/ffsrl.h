@@ -396,7 +396,8 @@ int32_t ffsrl_batch_class_split(const ffsrl_batch* b, int32_t cls, int32_t* bloc
 int32_t ffsrl_batch_set_class_block(ffsrl_batch* b, int32_t cls, int32_t block);
 /* Autotuner hook, how class cls's kernel fetches each thread's next tet record one loop
    trip ahead: 0 not at all, 1 into L1 (prefetch.global.L1), 2 into registers (block sizes
-   512 and 640, float32).  Results are unchanged.  A class whose envs are divided among
+   512 and 640, float32; a class of 768 whose block size the caller has not set goes to 512
+   for it).  Results are unchanged.  A class whose envs are divided among
    blocks takes any kind, and fetches in one way.  A kind the class's block size has no
    kernel for is refused and leaves the class as it was. */
 int32_t ffsrl_batch_set_class_prefetch(ffsrl_batch* b, int32_t cls, int32_t kind);
